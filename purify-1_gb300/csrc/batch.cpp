@@ -128,6 +128,7 @@ class BatchT final : public Batch {
   std::unique_ptr<Chan[]> chans_;
   std::vector<SizeGroup> groups_;
   int ntasks_ = 0, win_rows_ = 0, win_cols_ = 0;
+  DeviceBuffer taps_;  // FP64: stored tap weights of every channel (ApplyArgs::taps)
   Arena shared_;  // grouped task list, argument tables, padded and FFT grids
   size_t o_tasks_ = 0, o_task_base_ = 0, o_fwd_ = 0, o_adj_ = 0, o_folds_ = 0, o_io_ = 0,
          o_partial_ = 0, o_sq_ = 0, o_inv_ = 0, o_map_pix_ = 0, o_map_pad_ = 0, o_map_slot_ = 0,
@@ -429,10 +430,28 @@ BatchT<real>::BatchT(const BatchConfig &cfg) {
   adj_.resize(nch_);
   folds_.resize(nch_);
   io_.resize(nch_);
+  std::vector<size_t> o_taps(nch_);
+  if constexpr (sizeof(real) == 8) {
+    // stored taps of every channel, or of none (kTapTableShare)
+    size_t total = 0, free_b = 0, total_b = 0;
+    for (int c = 0; c < nch_; ++c) {
+      o_taps[c] = total;
+      total += sizeof(real) * 2 * size_t(J_) * size_t(chans_[c].S);
+    }
+    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    if (total > 0 && total <= free_b / kTapTableShare) {
+      taps_.alloc(total, &info_.device_bytes);
+      for (int c = 0; c < nch_; ++c)
+        cuda_check(launch_tap_table<real>(chans_[c].mem.template at<char>(chans_[c].o_frac), poly_,
+                                          J_, chans_[c].S, taps_.as<char>() + o_taps[c], stream_),
+                   "tap table");
+    }
+  }
   for (int c = 0; c < nch_; ++c) {
     Chan &ch = chans_[c];
     const Arena &m = ch.mem;
     ApplyArgs<real> a;
+    a.taps = taps_.get() ? taps_.as<char>() + o_taps[c] : nullptr;
     a.batches = m.at<int2>(ch.o_batches);
     a.lane_code = m.at<int32_t>(ch.o_lane);
     a.frac = m.at<char>(ch.o_frac);
@@ -569,6 +588,7 @@ void BatchT<real>::record(int mode) {
   const ChannelIO<real> *io = shared_.at<ChannelIO<real>>(o_io_);
   ApplyArgs<real> head;
   head.group_cells = cfg_group_;
+  head.taps = taps_.get();
   head.tasks = shared_.at<Task>(o_tasks_);
   head.order = shared_.at<int32_t>(o_order_);
   head.group_task_base = shared_.at<int32_t>(o_task_base_);

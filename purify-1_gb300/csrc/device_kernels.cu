@@ -133,6 +133,32 @@ __global__ void to_c128_kernel(const cplx<real> *__restrict__ src, double2 *__re
   }
 }
 
+// One slot per thread; a warp's 32 slots share one row of the table.
+template <typename real, int J, bool SUB>
+__global__ void tap_table_kernel(const cplx<real> *__restrict__ frac,
+                                 const __grid_constant__ PolyTable<real> poly, int64_t S,
+                                 real *__restrict__ taps) {
+  __shared__ real csm[SUB ? kMaxJ * kMaxSub * PolyCount<real>::value : 1];
+  if (SUB) {
+    stage_coefficients<real, J>(poly.u, poly.nsub_u, csm);
+    __syncthreads();
+  }
+  const int64_t s = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (s >= S) return;
+  const cplx<real> t = frac[s];
+  real ku[J], kv[J];
+  tap_weights<real, J, SUB>(poly.u, poly.nsub_u, fabs(t.x), ku, csm);
+  tap_weights<real, J, SUB>(poly.v, poly.nsub_v, t.y, kv, csm);
+  const int lane = int(s & 31);
+  real *row = taps + (s - lane) * (2 * J) + lane;
+  const bool flip = signbit(t.x);
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    row[32 * j] = flip ? -ku[j] : ku[j];
+    row[32 * (J + j)] = kv[j];
+  }
+}
+
 // Fixed-shape two-stage reduction: block b sums elements b*256+tid + k*stride
 // in ascending k, then a fixed tree; the second stage sums the block partials
 // in a fixed tree.  The result depends only on n.
@@ -419,6 +445,37 @@ cudaError_t launch_to_c128(const void *src, void *dst, int64_t n, cudaStream_t s
       static_cast<const cplx<real> *>(src), static_cast<double2 *>(dst), n);
   return cudaGetLastError();
 }
+
+template <typename real>
+cudaError_t launch_tap_table(const void *frac, const PolyTable<real> &poly, int J, int64_t S,
+                             void *taps, cudaStream_t s) {
+  if (S == 0) return cudaSuccess;
+  const bool sub = poly.nsub_u > 1 || poly.nsub_v > 1;
+  const int blocks = int((S + 127) / 128);
+  const auto *f = static_cast<const cplx<real> *>(frac);
+  auto *o = static_cast<real *>(taps);
+  switch (J) {
+#define PG_TAPS(JJ)                                                            \
+  case JJ:                                                                     \
+    if (sub)                                                                   \
+      tap_table_kernel<real, JJ, true><<<blocks, 128, 0, s>>>(f, poly, S, o);  \
+    else                                                                       \
+      tap_table_kernel<real, JJ, false><<<blocks, 128, 0, s>>>(f, poly, S, o); \
+    return cudaGetLastError();
+    PG_TAPS(1)
+    PG_TAPS(2)
+    PG_TAPS(3)
+    PG_TAPS(4)
+    PG_TAPS(5)
+    PG_TAPS(6)
+    PG_TAPS(7)
+    PG_TAPS(8)
+#undef PG_TAPS
+  }
+  return cudaErrorInvalidValue;
+}
+template cudaError_t launch_tap_table<double>(const void *, const PolyTable<double> &, int, int64_t,
+                                              void *, cudaStream_t);
 
 template <typename real>
 cudaError_t launch_sq_norm(const void *x, int64_t n, double *partial, double *out,

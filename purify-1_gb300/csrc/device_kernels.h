@@ -21,6 +21,10 @@ struct ApplyArgs {
   const int2 *batches = nullptr;    // {first slot, kmax}
   const int32_t *lane_code = nullptr;  // item_pack per batch lane
   const void *frac = nullptr;       // S x (t_u, t_v); sign of t_u = the phase flip (-1)^(k_u + k_v)
+  // Tap weights of every slot (launch_tap_table), or null: the kernels then
+  // evaluate the polynomials at frac.  FP64 only; a grouped launch sets it
+  // for every operator or for none, and in its own arguments too.
+  const void *taps = nullptr;
   void *slot_out = nullptr;         // degrid output, S complex
   const void *slot_in = nullptr;    // grid input, S complex
   // When set, visibilities are read / written in caller order directly:
@@ -67,6 +71,16 @@ size_t degrid_smem_bytes(int precision_bytes, int J, int win_rows, int win_cols,
 size_t grid_smem_bytes(int precision_bytes, int J, int win_rows, int win_cols,
                        const LaunchShape &shape, bool user = false, int group = 1,
                        int nsub = 1);
+
+// Tap weights of S slots (a multiple of 32) from their fractions, 2 J values
+// per slot in the layout of ApplyArgs::taps, evaluated as the gridding
+// kernels evaluate them, the phase sign folded into the u taps.
+// A table of more than 1 / kTapTableShare of the free device memory is not
+// made; the kernels then evaluate the polynomials, with the same bits.
+constexpr size_t kTapTableShare = 4;
+template <typename real>
+cudaError_t launch_tap_table(const void *frac, const PolyTable<real> &poly, int J, int64_t S,
+                             void *taps, cudaStream_t s);
 
 // G: tiles of the grid -> visibilities.
 template <typename real>

@@ -235,6 +235,23 @@ __device__ __forceinline__ cplx<real> gather_vis(const cplx<real> *vin, int m, b
   return keep ? load_keep(vin + m, pol) : vin[m];
 }
 
+// Stored tap weights (ApplyArgs::taps): the 2 J taps of a slot, u then v, as
+// taps[(slot - lane) 2 J + 32 i + lane], so that each tap of a warp's 32
+// slots is one 256-byte line.  The phase sign is folded into the u taps;
+// negating them negates every product and sum exactly, so the kernels'
+// results are those of the polynomials bit for bit.
+template <typename real, int J>
+__device__ __forceinline__ const real *tap_row(const void *taps, size_t slot0, int lane) {
+  return static_cast<const real *>(taps) + slot0 * (2 * J) + lane;
+}
+template <typename real, int J>
+__device__ __forceinline__ void load_taps(const real *row, real (&ku)[J], real (&kv)[J]) {
+#pragma unroll
+  for (int j = 0; j < J; ++j) ku[j] = __ldcs(row + 32 * j);
+#pragma unroll
+  for (int j = 0; j < J; ++j) kv[j] = __ldcs(row + 32 * (J + j));
+}
+
 // Operator arguments of a task.  A single-operator launch reads them from the
 // kernel parameters; a grouped launch (several operators in one grid) from
 // the device table at a0.group, indexed by the task's channel.
@@ -284,7 +301,13 @@ __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-template <typename real, int J, int G, bool SUB, bool GROUP>
+//
+// TAB: the taps come from the table at ApplyArgs::taps instead of the
+// polynomials.  FP64 kernels are bound by the FP64 pipe (about 1/64 of the
+// FP32 rate): at J = 6 the polynomials are 102 of a visibility's 186 FP64
+// operations per direction.  A table of 96 bytes per slot is read at HBM
+// speed instead (FP32, at 48 bytes against 8, would become bound by it).
+template <typename real, int J, int G, bool SUB, bool GROUP, bool TAB = false>
 __global__ void __launch_bounds__(256) degrid_kernel(const ApplyArgs<real> a0,
                                                      const __grid_constant__ PolyTable<real> poly) {
   using C = cplx<real>;
@@ -343,7 +366,7 @@ __global__ void __launch_bounds__(256) degrid_kernel(const ApplyArgs<real> a0,
     for (int j = 0; j < CH && lb < nbt; ++j) {
       const size_t i = size_t(th.hdr[lb].x) + size_t(k) * kBatch + lane;
       const int e = (buf * CH + j) * 32 + lane;
-      cp_async_stream<sizeof(C)>(st_t + e, frac + i, pol);
+      if constexpr (!TAB) cp_async_stream<sizeof(C)>(st_t + e, frac + i, pol);
       if (user) cp_async_stream<4>(st_m + e, user + i, pol);
       if (++k >= th.hdr[lb].y) {
         k = 0;
@@ -378,10 +401,18 @@ __global__ void __launch_bounds__(256) degrid_kernel(const ApplyArgs<real> a0,
           for (int ju = 0; ju < JBU; ++ju) F[jv][ju] = blk[win_offset(jv, ju, WS, G)];
       }
       const int e = (buf * CH + j) * 32 + lane;
-      const C t = st_t[e];
       real ku[JBU], kv[JBV];
-      block_taps<real, J, group_u(G), SUB>(poly.u, poly.nsub_u, fabs(t.x), ku, csm);
-      block_taps<real, J, group_v(G), SUB>(poly.v, poly.nsub_v, t.y, kv, csm);
+      // the phase sign (-1)^(k_u + k_v) rides in the sign of t_u (TAB: in ku)
+      real sg = real(1);
+      if constexpr (TAB) {
+        load_taps<real, J>(tap_row<real, J>(a.taps, size_t(bt.x) + size_t(k) * kBatch, lane), ku,
+                           kv);
+      } else {
+        const C t = st_t[e];
+        block_taps<real, J, group_u(G), SUB>(poly.u, poly.nsub_u, fabs(t.x), ku, csm);
+        block_taps<real, J, group_v(G), SUB>(poly.v, poly.nsub_v, t.y, kv, csm);
+        sg = copysign(real(1), t.x);
+      }
       C sum{0, 0};
 #pragma unroll
       for (int jv = 0; jv < JBV; ++jv) {
@@ -390,8 +421,6 @@ __global__ void __launch_bounds__(256) degrid_kernel(const ApplyArgs<real> a0,
         for (int ju = 0; ju < JBU; ++ju) row = fma2(splat(ku[ju]), F[jv][ju], row);
         sum = fma2(splat(kv[jv]), row, sum);
       }
-      // the phase sign (-1)^(k_u + k_v) rides in the sign of t_u
-      const real sg = copysign(real(1), t.x);
       const C y{sg * sum.x, sg * sum.y};
       // Lanes past their item's end compute on null slots: 0 in slot order,
       // nothing in caller order.
@@ -430,7 +459,9 @@ struct GridAhead {
   static constexpr int index_lead = narrow ? 3 : 1;
 };
 
-template <typename real, int J, int G, bool SUB, bool GROUP, bool CALLER = false>
+// TAB: stored taps, as in degrid_kernel.
+template <typename real, int J, int G, bool SUB, bool GROUP, bool CALLER = false,
+          bool TAB = false>
 __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
                                                    const __grid_constant__ PolyTable<real> poly) {
   using C = cplx<real>;
@@ -521,7 +552,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
       for (int i = 0; i < IL; ++i) mr[i] = user ? next_index() : -1;
     }
     auto prefetch = [&](C &t, C &y) {
-      t = stream_load(frac + slot(plb, pk));
+      if constexpr (!TAB) t = stream_load(frac + slot(plb, pk));
       if constexpr (IL == 1) {
         y = value_at(plb, pk, mq);
         adv(plb, pk);
@@ -557,13 +588,17 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
       }
       if (plb < nbt) prefetch(tq[D - 1], yq[D - 1]);
       // Null slots hold a zero visibility, so they add nothing.  The phase
-      // sign (-1)^(k_u + k_v) rides in the sign of t_u.
-      const real sg = copysign(real(1), t.x);
-      const real zr = sg * yv.x, zi = sg * yv.y;
+      // sign (-1)^(k_u + k_v) rides in the sign of t_u (TAB: in ku).
+      real sg = real(1);
       real ku[JBU], kv[JBV];
-      block_taps<real, J, group_u(G), SUB>(poly.u, poly.nsub_u, fabs(t.x), ku, csm);
-      block_taps<real, J, group_v(G), SUB>(poly.v, poly.nsub_v, t.y, kv, csm);
-      const C z{zr, zi};
+      if constexpr (TAB) {
+        load_taps<real, J>(tap_row<real, J>(a.taps, slot(clb, ck) - lane, lane), ku, kv);
+      } else {
+        sg = copysign(real(1), t.x);
+        block_taps<real, J, group_u(G), SUB>(poly.u, poly.nsub_u, fabs(t.x), ku, csm);
+        block_taps<real, J, group_v(G), SUB>(poly.v, poly.nsub_v, t.y, kv, csm);
+      }
+      const C z{sg * yv.x, sg * yv.y};
 #pragma unroll
       for (int jv = 0; jv < JBV; ++jv) {
         const C az = mul2(z, splat(kv[jv]));
@@ -1126,6 +1161,12 @@ template <typename real, int J, int G, bool SUB, bool GROUP>
 cudaError_t launch_one(bool degrid, const ApplyArgs<real> &a, const PolyTable<real> &poly,
                        int ntasks, size_t smem, int threads, cudaStream_t s) {
   auto fn = degrid ? degrid_kernel<real, J, G, SUB, GROUP> : grid_kernel<real, J, G, SUB, GROUP>;
+  if constexpr (sizeof(real) == 8 && G == 1 && !SUB) {
+    // stored taps
+    if (a.taps)
+      fn = degrid ? degrid_kernel<real, J, G, false, GROUP, true>
+                  : grid_kernel<real, J, G, false, GROUP, false, true>;
+  }
   if constexpr (sizeof(real) == 4 && J < 6 && G == 1 && !GROUP) {
     // G^H gathering caller order at narrow supports: deeper prefetch
     if (!degrid && a.slot_user) fn = grid_kernel<real, J, G, SUB, GROUP, true>;
@@ -1142,7 +1183,8 @@ template <typename real, bool GROUP>
 cudaError_t launch_apply(bool degrid, const ApplyArgs<real> &a, const PolyTable<real> &poly,
                          int J, int ntasks, size_t smem, int threads, cudaStream_t s) {
   if (ntasks == 0) return cudaSuccess;
-  const bool sub = poly.nsub_u > 1 || poly.nsub_v > 1;
+  // stored taps: the table stands for the sub-segmented polynomials too
+  const bool sub = !a.taps && (poly.nsub_u > 1 || poly.nsub_v > 1);
 #define PG_CASE(JJ, GG)                                                                  \
   case JJ:                                                                               \
     return sub ? launch_one<real, JJ, GG, true, GROUP>(degrid, a, poly, ntasks, smem, threads, s) \
