@@ -24,12 +24,13 @@ struct FftArgs {
   int Nx = 0, Ny = 0, Nu = 0, Nv = 0, x0 = 0, y0 = 0;
   int ld = 0;                                // row stride of the grid in cells (0: Nu)
   const float *su = nullptr, *sv = nullptr;  // correction per column / row of the image
-  const void *tw_u = nullptr;                // float2 exp(-2 pi i m / Nu), m < Nu
+  const void *tw_u = nullptr;                // fft_twiddles(Nu)
 };
 
 // True when the fused row passes handle grids Nu wide.
 bool fft_rows_supported(int Nu);
-// exp(-2 pi i m / N) for m < N, FP64-generated, as interleaved float pairs.
+// The twiddles of an N-point transform's stages, FP64-generated, as interleaved
+// float pairs (N of them, in the layout that fft_kernels.cu names).
 std::vector<float> fft_twiddles(int N);
 // x (Ny x Nx) -> rows y0 ... of grid (Nv x Nu), row-transformed.
 cudaError_t launch_fft_rows_forward(const FftArgs &a, const void *x, void *grid, cudaStream_t s);
@@ -47,7 +48,7 @@ struct FftColArgs {
   const void *in = nullptr;
   void *out = nullptr;
   int Nv = 0, W = 0, ld = 0, y0 = 0, Ny = 0;
-  const void *tw_v = nullptr;  // float2 exp(-2 pi i m / Nv), m < Nv
+  const void *tw_v = nullptr;  // fft_twiddles(Nv)
   const void *chans = nullptr;
   const int *members = nullptr;
   int Nu = 0;
