@@ -709,10 +709,9 @@ def run_wproj(args):
         "device_bytes": info["device_bytes"], "factor_values": info["factor_values"],
         "clocks": clocks, "kernel_bytes": wbytes,
         "roofline": roofline_entry(kern, wbytes[kern], dur, peak, peak_kind, None, formula),
-        # own kernels per step: the forward row pass, w degrid, the compaction
-        # into caller order, the gather into slot order, w grid, fold, the
-        # inverse row pass (the 4096-row columns go through cuFFT)
-        "gpu_launches": 7 * args.steps,
+        # own kernels per step: the forward row pass, w degrid, w grid, fold,
+        # the inverse row pass (the 4096-row columns go through cuFFT)
+        "gpu_launches": 5 * args.steps,
     }
     # FP32 rows against the FP64 oracle on a row sample (rows are independent)
     try:

@@ -21,6 +21,7 @@
 #include "plan.h"
 #include "wkernels.h"
 #include "wplan.h"
+#include "wstrip_kernels.h"
 
 namespace pg {
 
@@ -168,6 +169,15 @@ class OperatorT final : public Operator {
   int fold_J_ = 0, fold_Jv_ = 0;
   DeviceBuffer wcode_, wfactor_, wfactors_, wchunks_, wtask_chunk_;
   int wchunk_values_ = 0;
+  // Row factors on the tensor-core kernels (FP32): the strip plan's state.
+  // Visibilities are read and written in caller order; ws->slots, where it
+  // is used (the normal operator), then holds them in caller order too.
+  bool strips_ = false;
+  int64_t strip_cells_ = 0;  // cells of all task windows
+  WStripArgs strip_args_;
+  WStripFoldArgs strip_fold_;
+  DeviceBuffer stasks_, sorder_, sgroup_oct_, sterms_, sowner_;
+  void init_strips(const WStripPlan &plan, int64_t &bytes);
   int64_t nnz_ = 0, occupied_ = 0, work_items_ = 0, factor_values_ = 0;
   void init_plain(const OperatorConfig &cfg, int64_t &bytes, AxisTiling &tu, AxisTiling &tv,
                   std::vector<int32_t> &tile_tasks);
@@ -333,6 +343,7 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   // split weights are applied to the slot-ordered buffer before G^H, and the
   // column walk reads its own slot order
   if (split_weights_ || walk_) fused_adjoint_ = false;
+  if (strips_) fused_forward_ = fused_adjoint_ = true;
   ntu_ = tu.n;
   ntv_ = tv.n;
   slot_stride_ = int64_t(win_rows_) * win_cols_;
@@ -428,14 +439,14 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   info_.fp64 = cfg.fp64;
   info_.kernel = cfg.kernel;
   info_.w_term = cfg.w_term;
-  info_.tasks = ntasks_;
+  info_.tasks = strips_ ? strip_args_.ntasks : ntasks_;
   info_.device_bytes = bytes;
   info_.kernel_fit_error = wmode_ ? 0.0 : fit.max_error;
   info_.nnz = nnz_;
   info_.occupied_cells = occupied_;
   info_.work_items = work_items_;
   info_.slots = S_;
-  info_.window_cells = slot_stride_;
+  info_.window_cells = strips_ ? strip_cells_ / strip_args_.ntasks : slot_stride_;
   info_.factor_values = factor_values_;
   info_.cell_group = group_;
   info_.walk_tasks = walk_ ? walk_ntasks_ : 0;
@@ -652,40 +663,65 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
   win_rows_ = plan.win_rows;
   win_cols_ = plan.win_cols;
   fold_J_ = fold_Jv_ = plan.Smax;
+  tu = plan.tu;
+  tv = plan.tv;
+  tile_tasks = plan.tile_tasks;
+  if constexpr (sizeof(real) == 4) {
+    // The tensor-core kernels wherever their windows fit in the scratch of
+    // the band kernels' (the sizes callers see stay those), which is always so
+    // but for grids of a few groups.  Measured on a 1024^2 image with 2 x 10^6
+    // rows of 4 to 24 taps: Phi 541 us with the band kernels, 336 with these;
+    // Phi^H 1043, 395.  With 5 x 10^4 rows: 80, 83; 144, 109.
+    WStripPlan strips;
+    if (M_ > 0 && build_wstrips(plan, int64_t(win_rows_) * win_cols_ * ntasks_, strips)) {
+      init_strips(strips, bytes);
+      strips_ = true;
+    }
+  }
   S_ = M_;
   unit_weights_ = false;
   // the reference's non-zeros (Ju Jv per plain row; the stored rows pad to S^2)
   nnz_ = rows_mode_ ? M_ * int64_t(cfg.Ju) * cfg.Jv : plan.taps;
   occupied_ = 0;
   work_items_ = M_;
-  std::vector<C> wt(M_);
-  for (int64_t i = 0; i < M_; ++i)
-    wt[i] = C(real(plan.weight[i].real()), real(plan.weight[i].imag()));
-  weight_.alloc(sizeof(C) * std::max<int64_t>(M_, 1), &bytes);
-  weight_.upload(wt.data(), sizeof(C) * M_, stream_);
-  wcode_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
-  wcode_.upload(plan.code.data(), sizeof(int32_t) * M_, stream_);
-  wfactor_.alloc(sizeof(int64_t) * std::max<int64_t>(M_, 1), &bytes);
-  wfactor_.upload(plan.factor.data(), sizeof(int64_t) * M_, stream_);
-  slot_user_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
-  slot_user_.upload(plan.slot_user.data(), sizeof(int32_t) * M_, stream_);
-  user_slot_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
-  user_slot_.upload(plan.user_slot.data(), sizeof(int32_t) * M_, stream_);
-  tasks_.alloc(sizeof(Task) * std::max<size_t>(plan.tasks.size(), 1), &bytes);
-  tasks_.upload(plan.tasks.data(), sizeof(Task) * plan.tasks.size(), stream_);
-  task_order_.alloc(sizeof(int32_t) * std::max<size_t>(plan.task_order.size(), 1), &bytes);
-  task_order_.upload(plan.task_order.data(), sizeof(int32_t) * plan.task_order.size(), stream_);
-  wchunks_.alloc(sizeof(WChunk) * std::max<size_t>(plan.chunks.size(), 1), &bytes);
-  wchunks_.upload(plan.chunks.data(), sizeof(WChunk) * plan.chunks.size(), stream_);
-  wtask_chunk_.alloc(sizeof(int32_t) * plan.task_chunk.size(), &bytes);
-  wtask_chunk_.upload(plan.task_chunk.data(), sizeof(int32_t) * plan.task_chunk.size(), stream_);
+  // state of the band kernels (the strip plan's terms carry theirs)
+  std::vector<C> wt;
+  if (!strips_) {
+    wt.resize(M_);
+    for (int64_t i = 0; i < M_; ++i)
+      wt[i] = C(real(plan.weight[i].real()), real(plan.weight[i].imag()));
+    weight_.alloc(sizeof(C) * std::max<int64_t>(M_, 1), &bytes);
+    weight_.upload(wt.data(), sizeof(C) * M_, stream_);
+    wcode_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
+    wcode_.upload(plan.code.data(), sizeof(int32_t) * M_, stream_);
+    wfactor_.alloc(sizeof(int64_t) * std::max<int64_t>(M_, 1), &bytes);
+    wfactor_.upload(plan.factor.data(), sizeof(int64_t) * M_, stream_);
+    slot_user_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
+    slot_user_.upload(plan.slot_user.data(), sizeof(int32_t) * M_, stream_);
+    user_slot_.alloc(sizeof(int32_t) * std::max<int64_t>(M_, 1), &bytes);
+    user_slot_.upload(plan.user_slot.data(), sizeof(int32_t) * M_, stream_);
+    tasks_.alloc(sizeof(Task) * std::max<size_t>(plan.tasks.size(), 1), &bytes);
+    tasks_.upload(plan.tasks.data(), sizeof(Task) * plan.tasks.size(), stream_);
+    task_order_.alloc(sizeof(int32_t) * std::max<size_t>(plan.task_order.size(), 1), &bytes);
+    task_order_.upload(plan.task_order.data(), sizeof(int32_t) * plan.task_order.size(), stream_);
+    wchunks_.alloc(sizeof(WChunk) * std::max<size_t>(plan.chunks.size(), 1), &bytes);
+    wchunks_.upload(plan.chunks.data(), sizeof(WChunk) * plan.chunks.size(), stream_);
+    wtask_chunk_.alloc(sizeof(int32_t) * plan.task_chunk.size(), &bytes);
+    wtask_chunk_.upload(plan.task_chunk.data(), sizeof(int32_t) * plan.task_chunk.size(), stream_);
+  }
   wchunk_values_ = plan.chunk_values;
   factor_values_ = plan.factor_count;
   cuda_check(cudaStreamSynchronize(stream_), "upload");
   // Row factors, FP64-generated, uploaded in chunks of rows.  Two values of
   // tail: the G^H staging copies read whole 16-byte pieces.
-  wfactors_.alloc(sizeof(C) * (plan.factor_count + 2), &bytes);
-  cuda_check(cudaMemset(wfactors_.get(), 0, sizeof(C) * (plan.factor_count + 2)), "memset");
+  // The strip kernels form addresses up to 48 values past a row's factors and
+  // 16 before them (for copies of nothing): the strip plan's offsets start at
+  // kStripSlack, and as many values follow the last.
+  const int64_t slack = strips_ ? kStripSlack : 0;
+  wfactors_.alloc(sizeof(C) * (plan.factor_count + 2 * slack + 2), &bytes);
+  strip_args_.factors = wfactors_.as<C>() + slack;
+  cuda_check(cudaMemset(wfactors_.get(), 0, sizeof(C) * (plan.factor_count + 2 * slack + 2)),
+             "memset");
   const int64_t chunk_rows = 1 << 20;
   std::vector<std::complex<real>> buf;
   for (int64_t i0 = 0; i0 < M_; i0 += chunk_rows) {
@@ -694,13 +730,45 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
     const int64_t f1 = i1 < M_ ? plan.factor[i1] : plan.factor_count;
     buf.resize(size_t(f1 - f0));
     wplan_factors<real>(plan, i0, i1, buf.data());
-    cuda_check(cudaMemcpy(wfactors_.as<C>() + f0, buf.data(), sizeof(C) * (f1 - f0),
+    cuda_check(cudaMemcpy(wfactors_.as<C>() + slack + f0, buf.data(), sizeof(C) * (f1 - f0),
                           cudaMemcpyHostToDevice),
                "factor upload");
   }
-  tu = plan.tu;
-  tv = plan.tv;
-  tile_tasks = plan.tile_tasks;
+}
+
+template <typename real>
+void OperatorT<real>::init_strips(const WStripPlan &plan, int64_t &bytes) {
+  auto put = [&](DeviceBuffer &b, const auto &v) {
+    const size_t n = sizeof(v[0]) * v.size();
+    b.alloc(n, &bytes);
+    b.upload(v.data(), n, stream_);
+  };
+  put(stasks_, plan.tasks);
+  put(sorder_, plan.order);
+  put(sgroup_oct_, plan.group_oct);
+  put(sterms_, plan.terms);
+  put(sowner_, plan.owner);
+  cuda_check(cudaStreamSynchronize(stream_), "upload");  // the plan's arrays are pageable
+  WStripArgs &a = strip_args_;
+  a.tasks = stasks_.as<WStripTask>();
+  a.order = sorder_.as<int32_t>();
+  a.group_oct = sgroup_oct_.as<int32_t>();
+  a.terms = sterms_.as<WTerm>();
+  a.ntasks = int(plan.tasks.size());
+  strip_cells_ = plan.window_cells;
+  a.Nu = Nu_;
+  a.Nv = Nv_;
+  a.tiles = plan.tiles;
+  a.rows = plan.rows;
+  WStripFoldArgs &f = strip_fold_;
+  f.tasks = a.tasks;
+  f.owner = sowner_.as<int2>();
+  f.strips = plan.strips;
+  f.cols = plan.cols;
+  f.tiles = plan.tiles;
+  f.rows = plan.rows;
+  f.Nu = Nu_;
+  f.Nv = Nv_;
 }
 
 template <typename real>
@@ -754,6 +822,15 @@ void OperatorT<real>::release(cudaStream_t user) {
 
 template <typename real>
 void OperatorT<real>::degrid_slots(const void *grid, void *caller_vis) {
+  if (strips_) {
+    WStripArgs a = strip_args_;
+    a.grid = grid;
+    a.vis_out = caller_vis ? caller_vis : ws_->slots;
+    mark_begin(kDegrid);
+    cuda_check(launch_wstrip_degrid(a, ws_->stream), "w degrid");
+    mark_end(kDegrid);
+    return;
+  }
   if (wmode_) {
     WArgs<real> w;
     w.grid = grid;
@@ -814,6 +891,21 @@ void OperatorT<real>::grid_slots(void *grid, const void *caller_vis) {
 template <typename real>
 void OperatorT<real>::grid_core(void *grid, const void *vis, const int32_t *slot_user,
                                 void *windows) {
+  if (strips_) {
+    WStripArgs a = strip_args_;
+    a.vis_in = vis;
+    a.windows = windows;
+    mark_begin(kGrid);
+    cuda_check(launch_wstrip_grid(a, ws_->stream), "w grid");
+    mark_end(kGrid);
+    WStripFoldArgs f = strip_fold_;
+    f.windows = windows;
+    f.grid = grid;
+    mark_begin(kFold);
+    cuda_check(launch_wstrip_fold(f, ws_->stream), "fold");
+    mark_end(kFold);
+    return;
+  }
   if (wmode_) {
     WArgs<real> w;
     w.tilebuf = windows;
@@ -1185,7 +1277,7 @@ template <typename real>
 int64_t OperatorT<real>::no_alloc_bytes() const {
   auto up = [](int64_t b) { return (b + 255) / 256 * 256; };
   return up(int64_t(sizeof(C)) * slot_stride_ * std::max(ntasks_, 1)) +
-         (fused_adjoint_ ? 0 : up(int64_t(sizeof(C)) * std::max<int64_t>(S_, 1)));
+         (fused_adjoint_ && !wmode_ ? 0 : up(int64_t(sizeof(C)) * std::max<int64_t>(S_, 1)));
 }
 
 template <typename real>

@@ -81,6 +81,32 @@ struct WChunk {
 constexpr int kWChunkVis = 64;
 constexpr int kWChunkValues = 1024;
 
+// Strip plan of the tensor-core row kernels (wplan.h WStripPlan).
+constexpr int kStripRows = 16;  // rows of a strip: two blocks of 8
+constexpr int kStripCols = 8;   // columns of a group
+constexpr int kOctTerms = 8;
+// One factor pair of a row: A at factors[a], S complex values, B at
+// factors[a + b_off]; visibility m of the caller (-1: unused) and its weight,
+// phase sign folded in.  first_tap packs the row's first tap inside its
+// block of 8 x 8 cells (row | column << 4), the support S << 8, and how many
+// terms of the same row start here (1 to 3; 0: a later term of a row) << 16.
+// blocks: of its oct, the block rows reached | block columns << 4 | the half
+// of the strip << 8; bit 12: the oct's other four terms are unused.
+struct WTerm {
+  int64_t a;
+  int32_t b_off, m;
+  float wx, wy;
+  int32_t first_tap, blocks;
+};
+struct WStripTask {
+  int64_t window;           // first cell of the task's window in the scratch
+  int32_t P, Q;             // grid row and column of the window's first cell
+  int32_t groups;           // column groups walked
+  int32_t width;            // columns of the window
+  int32_t oct0;             // first entry of group_oct (groups + 1 of them)
+  int32_t pad;
+};
+
 // Work item encoding: .x = first visibility (plan order), .y = lp | lq << 8 |
 // count << 16 with (lp, lq) the base cell relative to the tile origin.  An
 // item with count 0 is padding.

@@ -233,6 +233,207 @@ WPlan build_wplan(const WPlanRequest &rq) {
   return P;
 }
 
+bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
+  WStripPlan W;
+  const int64_t M = plan.M;
+  W.tiles = (plan.Smax + 7 + 7) / 8;
+  W.rows = plan.Smax + kStripRows - 1;
+  W.strips = (plan.Nv + kStripRows - 1) / kStripRows;
+  W.cols = (plan.Nu + kStripCols - 1) / kStripCols;
+  const int64_t ngroups = int64_t(W.strips) * W.cols;
+
+  // Sort key of a row inside its group: half of the strip, then blocks of 8
+  // rows and columns reached, most first.
+  std::vector<int32_t> group(M);
+  std::vector<uint16_t> key(M), start(M);
+  std::vector<int32_t> tile(M);
+  for (size_t k = 0; k < plan.tasks.size(); ++k)
+    for (int32_t i = plan.tasks[k].batch_begin; i < plan.tasks[k].batch_end; ++i)
+      tile[i] = int32_t(k);
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < M; ++i) {
+    const int32_t code = plan.code[i];
+    const int S = wrow_support(code);
+    const int p = plan.tasks[tile[i]].P + (code & 0xff), q = plan.tasks[tile[i]].Q + ((code >> 8) & 0xff);
+    group[i] = (p / kStripRows) * W.cols + q / kStripCols;
+    const int half = (p % kStripRows) / 8, dv = p % 8, du = q % 8;
+    const int tv = (dv + S + 7) / 8, tu = (du + S + 7) / 8;
+    start[i] = uint16_t(dv | (du << 4));
+    key[i] = uint16_t((half << 8) | ((15 - tv) << 4) | (15 - tu));
+  }
+  // Stable counting sort by group, then a sort of each group by key.
+  std::vector<int64_t> first(ngroups + 1, 0);
+  for (int64_t i = 0; i < M; ++i) ++first[group[i] + 1];
+  for (int64_t g = 0; g < ngroups; ++g) first[g + 1] += first[g];
+  std::vector<int32_t> order(M);
+  {
+    std::vector<int64_t> fill(first.begin(), first.end() - 1);
+    for (int64_t i = 0; i < M; ++i) order[fill[group[i]]++] = int32_t(i);
+  }
+#pragma omp parallel for schedule(dynamic, 256)
+  for (int64_t g = 0; g < ngroups; ++g)
+    std::stable_sort(order.begin() + first[g], order.begin() + first[g + 1],
+                     [&](int32_t x, int32_t y) { return key[x] < key[y]; });
+
+  // Octs of every group: the terms of a row stay together, an oct stays in
+  // one half.  Rows are named by their position in the new order.
+  std::vector<int64_t> factor(M);
+  int64_t off = 0;
+  for (int64_t r = 0; r < M; ++r) {
+    factor[r] = off;
+    off += int64_t(2) * wrow_rank(plan.code[order[r]]) * wrow_support(plan.code[order[r]]);
+  }
+  std::vector<int32_t> goct(ngroups + 1, 0);  // first oct of each group
+  std::vector<int64_t> cost(ngroups, 0);
+  const WTerm none{0, 0, -1, 0.f, 0.f, 0, 0};
+  for (int64_t g = 0; g < ngroups; ++g) {
+    int used = kOctTerms, half = -1;
+    int32_t *oct = nullptr;
+    for (int64_t r = first[g]; r < first[g + 1]; ++r) {
+      const int32_t i = order[r], code = plan.code[i];
+      const int S = wrow_support(code), rank = wrow_rank(code);
+      if (rank == 0) continue;  // no tap is nonzero
+      if (used + rank > kOctTerms || half != (key[i] >> 8)) {
+        half = key[i] >> 8;
+        if (W.octs.size() >= size_t(INT32_MAX) / kOctTerms) return false;
+        W.octs.push_back(0);
+        W.terms.insert(W.terms.end(), kOctTerms, none);
+        oct = &W.octs.back();
+        used = 0;
+      }
+      const int tv = std::max(*oct & 15, 15 - ((key[i] >> 4) & 15));
+      const int tu = std::max((*oct >> 4) & 15, 15 - (key[i] & 15));
+      for (int e = 0; e < rank; ++e) {
+        WTerm &t = W.terms[(W.octs.size() - 1) * kOctTerms + used + e];
+        t.a = factor[r] + int64_t(e) * S;
+        t.b_off = rank * S;
+        t.m = plan.slot_user[i];
+        t.wx = float(plan.weight[i].real());
+        t.wy = float(plan.weight[i].imag());
+        t.first_tap = start[i] | (S << 8) | ((e == 0 ? rank : 0) << 16);
+      }
+      used += rank;
+      *oct = tv | (tu << 4) | (half << 8) | (used << 12);
+    }
+    for (int32_t o = goct[g]; o < int32_t(W.octs.size()); ++o)
+      for (int k = 0; k < kOctTerms; ++k)
+        W.terms[size_t(o) * kOctTerms + k].blocks =
+            (W.octs[o] & 0xfff) | (k < 4 && (W.octs[o] >> 12) <= 4 ? 1 << 12 : 0);
+    goct[g + 1] = int32_t(W.octs.size());
+    for (int32_t o = goct[g]; o < goct[g + 1]; ++o)
+      cost[g] += int64_t(W.octs[o] & 15) * ((W.octs[o] >> 4) & 15);
+  }
+
+  // Tasks: runs of groups of one strip, cut at gaps (where the columns a
+  // window carries past its last group would all be empty) and at a bound on
+  // the work (in blocks of an oct); a group above the bound is split.  A
+  // task's window is tail columns wider than its groups, which cost about as
+  // much as a few octs, so the bound gives kMinWork to a task once that
+  // leaves every SM its 7 CTAs, and three tasks to a warp of G^H (12 an SM)
+  // beyond that.  It grows until the windows fit.
+  int64_t total = 0;
+  for (int64_t g = 0; g < ngroups; ++g) total += cost[g] + 4;
+  const int tail = kStripCols * (W.tiles - 1);
+  auto cut = [&](int64_t bound) {
+    W.tasks.clear();
+    W.group_oct.clear();
+    W.owner.assign(ngroups, int2_t{0, 0});
+    W.window_cells = 0;
+    auto add = [&](int s, int c, int n, int32_t o0, int32_t o1) {
+      WStripTask t{};
+      t.P = s * kStripRows;
+      t.Q = c * kStripCols;
+      t.groups = n;
+      t.width = n * kStripCols + tail;
+      t.window = W.window_cells;
+      t.oct0 = int32_t(W.group_oct.size());
+      W.window_cells += int64_t(t.width) * W.rows;
+      W.group_oct.push_back(o0);
+      for (int k = 0; k < n; ++k)
+        W.group_oct.push_back(n == 1 ? o1 : goct[int64_t(s) * W.cols + c + k + 1]);
+      const int32_t id = int32_t(W.tasks.size());
+      W.tasks.push_back(t);
+      for (int k = 0; k < n; ++k) {
+        int2_t &w = W.owner[int64_t(s) * W.cols + c + k];
+        if (w.x == w.y) w.x = id;
+        w.y = id + 1;
+      }
+    };
+    for (int s = 0; s < W.strips; ++s)
+      for (int c = 0; c < W.cols;) {
+        const int64_t g0 = int64_t(s) * W.cols;
+        if (goct[g0 + c] == goct[g0 + c + 1]) {
+          ++c;
+          continue;
+        }
+        if (cost[g0 + c] > bound && goct[g0 + c + 1] - goct[g0 + c] > 1) {
+          // parts of one group
+          const int32_t a = goct[g0 + c], n = goct[g0 + c + 1] - a;
+          const int32_t parts = int32_t(std::min<int64_t>(n, (cost[g0 + c] + bound - 1) / bound));
+          for (int32_t k = 0; k < parts; ++k)
+            add(s, c, 1, a + int32_t(int64_t(n) * k / parts), a + int32_t(int64_t(n) * (k + 1) / parts));
+          ++c;
+          continue;
+        }
+        int e = c, gap = 0, last = c;
+        int64_t work = 0;
+        while (e < W.cols && gap < W.tiles) {
+          const int64_t g = g0 + e;
+          const bool empty = goct[g] == goct[g + 1];
+          if (!empty) {
+            if (e > c && (work + cost[g] > bound || cost[g] > bound)) break;
+            last = e;
+          }
+          work += cost[g] + 4;
+          gap = empty ? gap + 1 : 0;
+          ++e;
+        }
+        add(s, c, last - c + 1, goct[g0 + c], goct[g0 + last + 1]);
+        c = last + 1;
+      }
+  };
+  constexpr int64_t kMinWork = 256;
+  const int64_t most = total / (152 * 12 * 3), few = std::min(kMinWork, total / (152 * 7));
+  for (int64_t bound = std::max<int64_t>(64, std::max(most, few));; bound += bound / 8 + 1) {
+    cut(bound);
+    if (W.window_cells <= max_cells) break;
+    if (bound > total) return false;
+  }
+  W.order.resize(W.tasks.size());
+  std::iota(W.order.begin(), W.order.end(), 0);
+  std::vector<int64_t> tcost(W.tasks.size(), 0);
+  for (size_t k = 0; k < W.tasks.size(); ++k) {
+    const WStripTask &t = W.tasks[k];
+    tcost[k] = 4 * t.groups;
+    for (int32_t o = W.group_oct[t.oct0]; o < W.group_oct[t.oct0 + t.groups]; ++o)
+      tcost[k] += int64_t(W.octs[o] & 15) * ((W.octs[o] >> 4) & 15);
+  }
+  std::stable_sort(W.order.begin(), W.order.end(),
+                   [&](int32_t x, int32_t y) { return tcost[x] > tcost[y]; });
+
+  // The plan's rows in strip order.
+  auto permute = [&](auto &v) {
+    auto old = v;
+#pragma omp parallel for schedule(static)
+    for (int64_t r = 0; r < M; ++r) v[r] = old[order[r]];
+  };
+  permute(plan.code);
+  permute(plan.weight);
+  permute(plan.slot_user);
+  permute(plan.gen_u);
+  permute(plan.gen_v);
+  permute(plan.gen_w);
+  permute(plan.gen_jw);
+  plan.factor = factor;
+  for (int64_t r = 0; r < M; ++r) plan.user_slot[plan.slot_user[r]] = int32_t(r);
+  plan.tasks.clear();
+  plan.task_order.clear();
+  plan.chunks.clear();
+  plan.task_chunk.assign(1, 0);
+  out = std::move(W);
+  return true;
+}
+
 template <typename T>
 void wplan_factors(const WPlan &P, int64_t i0, int64_t i1, std::complex<T> *out) {
   const int J = P.J;

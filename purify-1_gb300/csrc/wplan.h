@@ -42,6 +42,10 @@ struct WPlanRequest {
   int Ju = 4, Jv = 4;
 };
 
+struct int2_t {
+  int32_t x, y;
+};
+
 struct WPlan {
   int64_t M = 0;
   int Nu = 0, Nv = 0, J = 0, Smax = 0;
@@ -73,6 +77,37 @@ struct WPlan {
 };
 
 WPlan build_wplan(const WPlanRequest &rq);
+
+// The strip plan of the tensor-core row kernels (wstrip_kernels.h; complex
+// <float>).  The grid is cut into strips of kStripRows rows and groups of
+// kStripCols columns; a row belongs to the group of its first tap's cell.  A
+// task is one warp's work: a run of groups of one strip, walked from left to
+// right, or, where one group holds too many rows, a part of it.
+//
+// A row's nonzero factor pairs (A_e, B_e) are its terms.  The kernels take
+// terms eight at a time (an oct).  The terms of one oct start in the same
+// half (8 rows) of the strip, and their taps reach `tv` blocks of 8 rows and
+// `tu` blocks of 8 columns from there; a group's rows are sorted by half, tv
+// and tu, so that an oct's blocks are few.  The terms of a row share an oct.
+// Unused terms have support 0.
+struct WStripPlan {
+  int tiles = 0;  // largest tv or tu: ceil((Smax + 7) / 8)
+  int rows = 0;   // rows of a task's window: Smax + kStripRows - 1
+  int strips = 0, cols = 0;          // strips and column groups of the grid
+  std::vector<WStripTask> tasks;     // by strip, then column
+  std::vector<int32_t> order;        // launch order: most work first
+  std::vector<int32_t> group_oct;    // per task its groups + 1 offsets into octs
+  std::vector<int32_t> octs;         // tv | tu << 4 | half << 8 | terms << 12
+  std::vector<WTerm> terms;          // 8 per oct
+  std::vector<int2_t> owner;         // strips x cols: tasks [x, y) that hold the group
+  int64_t window_cells = 0;          // complex cells of all task windows
+};
+
+// Reorders the rows of `plan` into strip order (its tasks and chunks, which
+// name rows by their old order, are emptied) and builds the strip plan, with
+// task windows of at most max_cells complex cells in all.  Returns false, with
+// `plan` untouched, where that is not possible.
+bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out);
 
 // Fields of a row code: the support S and the mask of stored terms (bit r:
 // term r of the sample matrix is nonzero); the rank is the mask's popcount.

@@ -1,0 +1,138 @@
+"""The tensor-core row kernels (FP32 w-projection rows, supports of 9 to 32
+taps, Ju != Jv) at the edges of their blocks, against the FP64 oracle.
+
+Tolerance (relative L2): 2e-6.  Operands are split so that a product keeps
+about 2^-23 of itself; with sums of a few hundred terms of random sign the
+result is within a few times that, 5e-7, and a lost or misplaced tap would
+show at 1e-3.  Non-finite values stay inside the footprints they belong to;
+the finite rest is held to the same tolerance."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from purify_gb300 import synthetic
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-6
+
+
+def _w(rng, M, N, cell=1.0):
+    return rng.uniform(-12, 12, M) * 60.0 * 60.0 * 180.0 / cell / N / np.pi
+
+
+def _check(pg, oracle_mod, torch, args, kw, okw, ny, nx, seed):
+    M = args[0].size
+    rng = np.random.default_rng(seed)
+    op = pg.MeasurementOperator(*args, ny, nx, 2.0, power_iters=0, precision="fp32", **kw)
+    ref = oracle_mod.Operator(*args, ny, nx, 2.0, **okw)
+    x = rng.standard_normal(ny * nx) + 1j * rng.standard_normal(ny * nx)
+    y = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    xd = torch.from_numpy(x).to(torch.complex64).cuda()
+    yd = torch.from_numpy(y).to(torch.complex64).cuda()
+    f, a = op.forward(xd), op.adjoint(yd)
+    assert rel_l2(f.cpu().numpy(), ref.forward(x)) < TOL
+    assert rel_l2(a.cpu().numpy(), ref.adjoint(y)) < TOL
+    assert torch.equal(op.normal(xd), op.adjoint(op.forward(xd)))
+    assert torch.equal(op.forward(xd), f) and torch.equal(op.adjoint(yd), a)
+
+
+# supports S = Jw + 3 on both sides of a change in the number of 8-cell blocks
+# (S + 7 = 8 k), one visibility, a dense cell, odd and unequal sizes
+@pytest.mark.parametrize("Jw,M,ny,nx,dense", [
+    (1, 1, 32, 32, False), (6, 2000, 33, 50, False), (7, 3000, 48, 31, False),
+    (14, 1500, 64, 40, True), (15, 700, 37, 64, False), (22, 1000, 48, 36, False),
+    (29, 800, 31, 62, True)])
+def test_w_rows_at_block_edges(pg, oracle_mod, cuda, Jw, M, ny, nx, dense):
+    rng = np.random.default_rng(Jw)
+    u, v = rng.uniform(-nx, nx, M), rng.uniform(-ny, ny, M)
+    if dense:
+        u[: M // 2], v[: M // 2] = 3.25 + 0.5 * rng.random(M // 2), -5.75 + 0.5 * rng.random(M // 2)
+    w = _w(rng, M, 2 * nx)
+    wt = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    kw = dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=Jw)
+    _check(pg, oracle_mod, cuda, (u, v, w, wt), kw, kw, ny, nx, Jw)
+
+
+def test_mixed_supports_and_empty_stretches(pg, oracle_mod, cuda):
+    n, M = 128, 900  # sparse: tasks are cut at gaps
+    rng = np.random.default_rng(2)
+    u, v = synthetic.gaussian_core_uv(M, 2 * n, 2 * n, 0.2, seed=3)
+    u[:40], v[:40] = rng.uniform(-n, n, 40), rng.uniform(-n, n, 40)
+    w = _w(rng, M, 2 * n)
+    jw = rng.integers(1, 22, M).astype(np.int32)
+    kw = dict(kernel="kb", Ju=4, Jv=4, w_term=True, jw_rows=jw)
+    _check(pg, oracle_mod, cuda, (u, v, w, None), kw, kw, n, n, 5)
+
+
+@pytest.mark.parametrize("kernel,Ju,Jv", [("gauss", 3, 2), ("kb", 9, 9), ("gauss", 18, 18),
+                                          ("kb", 25, 25)])
+def test_plain_rows(pg, oracle_mod, cuda, kernel, Ju, Jv):
+    rng = np.random.default_rng(Ju)
+    M, ny, nx = 600, 48, 36
+    u, v = rng.uniform(-nx, nx, M), rng.uniform(-ny, ny, M)
+    kw = dict(kernel=kernel, Ju=Ju, Jv=Jv)
+    _check(pg, oracle_mod, cuda, (u, v, None, None), kw, kw, ny, nx, Ju)
+
+
+def test_largest_support(pg, cuda):
+    """G and G^H alone against the FP64 operator's: the image-plane correction
+    of so wide a Gaussian amplifies the FFT's own rounding past the tolerance."""
+    torch = cuda
+    rng = np.random.default_rng(32)
+    M, ny, nx = 600, 31, 62
+    u, v = rng.uniform(-nx, nx, M), rng.uniform(-ny, ny, M)
+    y = torch.from_numpy(rng.standard_normal(M) + 1j * rng.standard_normal(M)).cuda()
+    g = torch.from_numpy(rng.standard_normal(4 * ny * nx) + 1j * rng.standard_normal(4 * ny * nx))
+    out = {}
+    for prec, dt in (("fp32", torch.complex64), ("fp64", torch.complex128)):
+        op = pg.MeasurementOperator(u, v, None, None, ny, nx, 2.0, power_iters=0, kernel="gauss",
+                                    Ju=32, Jv=32, precision=prec)
+        gd = g.to(torch.complex64).to(dt).cuda()
+        vis, grid = torch.empty(M, dtype=dt, device="cuda"), torch.empty_like(gd)
+        op.degrid_into(gd, vis)
+        op.grid_into(y.to(torch.complex64).to(dt), grid)
+        out[prec] = vis.cpu().numpy(), grid.cpu().numpy()
+    for a, b in zip(out["fp32"], out["fp64"]):
+        assert rel_l2(a, b) < TOL
+
+
+def test_non_finite_values_stay_in_their_footprint(pg, cuda):
+    torch = cuda
+    n, M, S = 64, 400, 9
+    N = 2 * n
+    rng = np.random.default_rng(8)
+    u, v = rng.uniform(-20, 20, M), rng.uniform(-20, 20, M)
+    w = _w(rng, M, N)
+    op = pg.MeasurementOperator(u, v, w, None, n, n, 2.0, power_iters=0, kernel="kb", Ju=4, Jv=4,
+                                w_term=True, Jw=S - 3, precision="fp32")
+    y = torch.from_numpy(rng.standard_normal(M) + 1j * rng.standard_normal(M)).to(
+        torch.complex64).cuda()
+    grid0 = torch.empty(N * N, dtype=torch.complex64, device="cuda")
+    grid1 = torch.empty_like(grid0)
+    k = 7
+    q = np.mod(np.floor(u[k] - S / 2) + 1 + np.arange(S), N).astype(int)
+    p = np.mod(np.floor(v[k] - S / 2) + 1 + np.arange(S), N).astype(int)
+    inside = np.zeros((N, N), bool)
+    inside[np.ix_(p, q)] = True
+    y[k] = 0
+    op.grid_into(y, grid0)
+    for bad in (float("inf"), float("nan")):
+        y[k] = bad
+        op.grid_into(y, grid1)
+        g0, g1 = (t.cpu().numpy().reshape(N, N) for t in (grid0, grid1))
+        assert not np.isfinite(g1[inside]).any()
+        assert np.isfinite(g1[~inside]).all()
+        assert rel_l2(g1[~inside], g0[~inside]) < TOL
+    # G: a NaN cell reaches the visibilities whose rows hold it
+    vis0 = torch.empty(M, dtype=torch.complex64, device="cuda")
+    vis1 = torch.empty_like(vis0)
+    op.degrid_into(grid0, vis0)
+    pc, qc = 3, N - 2
+    grid0[pc * N + qc] = float("nan")
+    op.degrid_into(grid0, vis1)
+    hit = ((np.mod(qc - np.floor(u - S / 2) - 1, N) < S) &
+           (np.mod(pc - np.floor(v - S / 2) - 1, N) < S))
+    assert hit.any() and not hit.all()
+    f0, f1 = vis0.cpu().numpy(), vis1.cpu().numpy()
+    assert not np.isfinite(f1[hit]).any() and np.isfinite(f1[~hit]).all()
+    assert rel_l2(f1[~hit], f0[~hit]) < TOL
