@@ -399,14 +399,14 @@ BatchT<real>::BatchT(const BatchConfig &cfg) {
         g.fft = make_column_plan<real>(g.ld, g.Nv, stream_, &info_.device_bytes);
         g.fft_ok = true;
       }
-      const std::vector<float> twv = fft_twiddles(g.Nv);
+      const std::vector<float> twv = fft_twiddle_table(g.Nv);
       cuda_check(cudaMemcpyAsync(shared_.at<char>(g.o_twv), twv.data(), sizeof(float) * twv.size(),
                                  cudaMemcpyHostToDevice, stream_),
                  "upload");
       cuda_check(cudaMemcpyAsync(shared_.at<char>(g.o_members), g.chans.data(),
                                  sizeof(int) * g.chans.size(), cudaMemcpyHostToDevice, stream_),
                  "upload");
-      const std::vector<float> tw = fft_twiddles(g.Nu);
+      const std::vector<float> tw = fft_twiddle_table(g.Nu);
       cuda_check(cudaMemcpyAsync(shared_.at<char>(g.o_tw), tw.data(), sizeof(float) * tw.size(),
                                  cudaMemcpyHostToDevice, stream_),
                  "upload");
@@ -678,6 +678,7 @@ FftColArgs BatchT<real>::col_args(const SizeGroup &g, bool inverse) const {
   c.W = g.ld;
   c.ld = g.ld;
   c.tw_v = shared_.at<char>(g.o_twv);
+  c.tw_table = true;
   c.chans = shared_.at<char>(o_io_);
   c.members = shared_.at<int>(g.o_members);
   c.Nu = g.Nu;

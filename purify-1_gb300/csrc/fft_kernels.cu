@@ -162,6 +162,29 @@ __device__ __forceinline__ int sidx(int row, int n) {
   return row * NP + n + (n >> 5);
 }
 
+// Twiddles w^r, r = 1 ... R-1, of w = exp(-+2 pi i k / (Ns R)) from w, w^2
+// and w^4 (loaded from the table): the others as one product of two of them.
+template <int R>
+__device__ __forceinline__ void twiddle(float2 *v, const float2 (&w)[4]) {
+  // w^r from the loaded powers w^(2^e): the product over the set bits of r
+  float2 p[R];
+  p[1] = w[0];
+#pragma unroll
+  for (int r = 2; r < R; ++r) {
+    const int top = 31 - __clz(r), low = r - (1 << top);  // compile-time after unrolling
+    p[r] = low ? cmulf(p[low], w[top]) : w[top];
+  }
+#pragma unroll
+  for (int r = 1; r < R; ++r) v[r] = cmulf(v[r], p[r]);
+}
+
+// The twiddles of every stage after the first, loaded in the prologue
+// together with the first stage's data so that one load latency covers them.
+constexpr int kMaxStages = 4, kMaxQ = 8, kMaxPow = 4;
+struct TwiddleCache {
+  float2 w[kMaxStages][kMaxQ][kMaxPow];
+};
+
 // Radix of the stage with sub-transform length Ns: 16 while it divides the
 // rest, then the remainder (2, 4 or 8).
 template <int N, int Ns>
@@ -170,26 +193,72 @@ struct StageRadix {
   static constexpr int value = rem % 16 == 0 ? 16 : rem;
 };
 
-// The twiddles w^(r k), w = exp(-2 pi i / (Ns R)), r = 1 ... R-1, k < Ns, of
-// every stage after the first, each FP64-generated and rounded once: the
-// table of fft_twiddles, entry (r - 1) Ns + k of a stage from Ns - R0 on (R0
-// the first stage's radix; N - R0 values in all).  A CTA copies it into
-// shared memory while it waits for its input.  Products of a few loaded
-// powers, which this replaces, cost up to three roundings a twiddle and 4 to 11
-// complex products a butterfly: Phi of a 1024^2 image was 1.2e-7 off in the
-// 2-norm, 1.0e-7 with the table, and the four passes of its 2048^2 transforms
-// took 70 us, 65.5 with it.
+template <int N, int V, int Ns, int S, bool INV, int T = kFftThreads, bool COLIO = false>
+__device__ __forceinline__ void load_twiddles(TwiddleCache &c, const float2 *__restrict__ tw) {
+  constexpr int R = StageRadix<N, Ns>::value;
+  constexpr int NB = V * (N / R);
+  constexpr int Q = (NB + T - 1) / T;
+  static_assert(S < kMaxStages && Q <= kMaxQ, "twiddle cache size");
+  if constexpr (Ns > 1) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int flat = int(threadIdx.x) + q * T;
+      // the last stage of a column pass takes its butterflies column-fastest
+      const int j = (COLIO && Ns * R == N) ? flat / V : flat % (N / R);
+      const int step = (j % Ns) * (N / (Ns * R));
+#pragma unroll
+      for (int e = 0; e < kMaxPow; ++e) {
+        if ((1 << e) < R && flat < NB) {
+          float2 w = __ldg(tw + (step << e));
+          if (INV) w.y = -w.y;
+          c.w[S][q][e] = w;
+        }
+      }
+    }
+  }
+  if constexpr (Ns * R < N) load_twiddles<N, V, Ns * R, S + 1, INV, T, COLIO>(c, tw);
+}
+
+// The alternative: every twiddle w^(r k) of a stage, r = 1 ... R-1, k < Ns, from
+// a table in shared memory (fft_twiddle_table; entry (r - 1) Ns + k of a stage
+// from Ns - R0 on, R0 the first stage's radix), which a CTA copies while it
+// waits for its input.  It saves the products (4 to 11 complex products a
+// butterfly: the four passes of a 2048^2 grid take 65.5 us, 70 with the
+// cache) and their roundings (a transform is 10 to 20% closer to the exact
+// one).  Operators whose complex<double> host results are to keep their bits
+// use the cache.
+struct TwiddleTable {
+  const float2 *w;
+};
 template <int N, int T>
-__device__ __forceinline__ void copy_twiddles(float2 *tws, const void *tw) {
+__device__ __forceinline__ TwiddleTable copy_twiddles(float2 *tws, const void *tw) {
   constexpr int pieces = (N - StageRadix<N, 1>::value) / 2;  // of 16 bytes
   const float4 *src = static_cast<const float4 *>(tw);
   const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(tws));
   for (int k = threadIdx.x; k < pieces; k += T)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * k), "l"(src + k)
                  : "memory");
+  return TwiddleTable{tws};
+}
+template <int N, int Ns, int S, int R, bool INV>
+__device__ __forceinline__ void apply_twiddles(float2 *v, const TwiddleCache &tc, int q, int) {
+  twiddle<R>(v, tc.w[S][q]);
+}
+template <int N, int Ns, int S, int R, bool INV>
+__device__ __forceinline__ void apply_twiddles(float2 *v, const TwiddleTable &t, int, int k) {
+#pragma unroll
+  for (int r = 1; r < R; ++r) {
+    float2 w = t.w[Ns - StageRadix<N, 1>::value + (r - 1) * Ns + k];
+    if (INV) w.y = -w.y;
+    v[r] = cmulf(v[r], w);
+  }
+}
+__device__ __forceinline__ void await_twiddles(const TwiddleCache &) {}
+__device__ __forceinline__ void await_twiddles(const TwiddleTable &) {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// The stage with sub-transform length Ns of an N-point transform of V rows.  With
+// Stage S (sub-transform length Ns) of an N-point transform of V rows.  With
 // COLIO the V "rows" are
 // V adjacent columns of a grid with row stride a.ld starting at column row0:
 // the first and last stages take their butterflies column-fastest (thread
@@ -198,10 +267,11 @@ __device__ __forceinline__ void copy_twiddles(float2 *tws, const void *tw) {
 // first stage reads only rows a.y0 ... a.y0+a.Ny-1 (forward), the last writes
 // only those rows (inverse).  Otherwise the first and last stages go through
 // load_in / store_out.
-template <int N, int V, int Ns, bool INV, int PAD = 0, int T = kFftThreads, bool COLIO = false>
+template <int N, int V, int Ns, int S, bool INV, int PAD = 0, int T = kFftThreads,
+          bool COLIO = false, typename TW = TwiddleCache>
 __device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *__restrict__ in,
                                            float2 *__restrict__ out, float2 *sm,
-                                           const float2 *tws, int row0) {
+                                           const TW &tc, int row0) {
   constexpr int R = StageRadix<N, Ns>::value;
   constexpr bool FIRST = Ns == 1, LAST = Ns * R == N;
   constexpr int NB = V * (N / R);  // butterflies of the stage
@@ -237,14 +307,7 @@ __device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *__res
       const bool cm = COLIO && (FIRST || LAST);
       const int rr = cm ? flat % V : flat / (N / R), j = cm ? flat / V : flat % (N / R);
       const int k = j % Ns;
-      if constexpr (!FIRST) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 w = tws[Ns - StageRadix<N, 1>::value + (r - 1) * Ns + k];
-          if (INV) w.y = -w.y;
-          v[q][r] = cmulf(v[q][r], w);
-        }
-      }
+      if constexpr (!FIRST) apply_twiddles<N, Ns, S, R, INV>(v[q], tc, q, k);
       dft<R, INV>(v[q]);
       const int d = (j / Ns) * Ns * R + k;
 #pragma unroll
@@ -261,22 +324,28 @@ __device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *__res
     }
   }
   if constexpr (!LAST) {
-    if constexpr (FIRST) asm volatile("cp.async.wait_all;\n" ::: "memory");  // the twiddles
+    if constexpr (FIRST) await_twiddles(tc);
     __syncthreads();
-    run_stages<N, V, Ns * R, INV, PAD, T, COLIO>(a, in, out, sm, tws, row0);
+    run_stages<N, V, Ns * R, S + 1, INV, PAD, T, COLIO, TW>(a, in, out, sm, tc, row0);
   }
 }
 
-template <int N, int V, bool INV>
+template <int N, int V, bool INV, bool TABLE>
 __global__ void __launch_bounds__(kFftThreads, 4) fft_row_kernel(const FftArgs a,
                                                               const float2 *__restrict__ in,
                                                               float2 *__restrict__ out) {
   extern __shared__ float2 fft_sm[];
   dev::pdl_launch_next();
-  float2 *tws = fft_sm + V * (N + N / 32);
-  copy_twiddles<N, kFftThreads>(tws, a.tw_u);
+  if constexpr (TABLE) {
+    const TwiddleTable t = copy_twiddles<N, kFftThreads>(fft_sm + V * (N + N / 32), a.tw_u);
+    dev::pdl_wait();
+    run_stages<N, V, 1, 0, INV, 0, kFftThreads, false>(a, in, out, fft_sm, t, int(blockIdx.x) * V);
+    return;
+  }
+  TwiddleCache tc;
+  load_twiddles<N, V, 1, 0, INV>(tc, static_cast<const float2 *>(a.tw_u));
   dev::pdl_wait();  // `in` is the previous kernel's output
-  run_stages<N, V, 1, INV>(a, in, out, fft_sm, tws, int(blockIdx.x) * V);
+  run_stages<N, V, 1, 0, INV>(a, in, out, fft_sm, tc, int(blockIdx.x) * V);
 }
 
 // One size group of a batch: member blockIdx.y's arguments from the channel
@@ -300,9 +369,8 @@ __global__ void __launch_bounds__(kFftThreads, 4) fft_row_group_kernel(
   a.sv = c.sv;
   const float2 *in = static_cast<const float2 *>(INV ? c.work : c.x_in);
   float2 *out = static_cast<float2 *>(INV ? c.x_out : c.pad);
-  float2 *tws = fft_sm + V * (N + N / 32);
-  copy_twiddles<N, kFftThreads>(tws, tw);
-  run_stages<N, V, 1, INV>(a, in, out, fft_sm, tws, int(blockIdx.x) * V);
+  const TwiddleTable t = copy_twiddles<N, kFftThreads>(fft_sm + V * (N + N / 32), tw);
+  run_stages<N, V, 1, 0, INV, 0, kFftThreads, false>(a, in, out, fft_sm, t, int(blockIdx.x) * V);
 }
 
 // Column pass: V adjacent columns per CTA, so that every row of the block is
@@ -330,7 +398,7 @@ struct ColPad {
 
 // The column pass with its first and last stages on global memory directly
 // (run_stages COLIO): no copy-in and copy-out passes through shared memory.
-template <int N, int V, bool INV, int T, int MINB>
+template <int N, int V, bool INV, int T, int MINB, bool TABLE>
 __global__ void __launch_bounds__(T, MINB) fft_col_direct_kernel(const FftColArgs c) {
   extern __shared__ float2 fft_sm[];
   dev::pdl_launch_next();
@@ -346,19 +414,28 @@ __global__ void __launch_bounds__(T, MINB) fft_col_direct_kernel(const FftColArg
     a.y0 = io.y0;
     a.Ny = io.Ny;
   }
-  float2 *tws = fft_sm + V * (N + N / 32 + PAD);
-  copy_twiddles<N, T>(tws, c.tw_v);
+  if constexpr (TABLE) {
+    const TwiddleTable t = copy_twiddles<N, T>(fft_sm + V * (N + N / 32 + PAD), c.tw_v);
+    dev::pdl_wait();
+    run_stages<N, V, 1, 0, INV, PAD, T, true>(a, static_cast<const float2 *>(c.in),
+                                              static_cast<float2 *>(c.out), fft_sm, t, col0);
+    return;
+  }
+  TwiddleCache tc;
+  load_twiddles<N, V, 1, 0, INV, T, true>(tc, static_cast<const float2 *>(c.tw_v));
   dev::pdl_wait();  // c.in is the previous kernel's output
-  run_stages<N, V, 1, INV, PAD, T, true>(a, static_cast<const float2 *>(c.in),
-                                         static_cast<float2 *>(c.out), fft_sm, tws, col0);
+  run_stages<N, V, 1, 0, INV, PAD, T, true>(a, static_cast<const float2 *>(c.in),
+                                                   static_cast<float2 *>(c.out), fft_sm, tc,
+                                                   col0);
 }
 
 template <int N, bool INV>
 cudaError_t launch_cols(const FftColArgs &c, cudaStream_t s) {
   constexpr int V = col_block(N), T = col_threads(N);
   constexpr int PAD = ColPad<N, V>::value;
-  const size_t smem = sizeof(float2) * (size_t(V) * (N + N / 32 + PAD) + N);
-  auto fn = fft_col_direct_kernel<N, V, INV, T, T == 512 ? 1 : 2>;
+  const size_t smem = sizeof(float2) * (size_t(V) * (N + N / 32 + PAD) + (c.tw_table ? N : 0));
+  auto fn = c.tw_table ? fft_col_direct_kernel<N, V, INV, T, T == 512 ? 1 : 2, true>
+                       : fft_col_direct_kernel<N, V, INV, T, T == 512 ? 1 : 2, false>;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -387,8 +464,8 @@ constexpr int rows_per_cta(int N) { return N >= 4096 ? 1 : 4096 / N; }
 template <int N, bool INV>
 cudaError_t launch_rows(const FftArgs &a, const void *in, void *out, cudaStream_t s) {
   constexpr int V = rows_per_cta(N);
-  const size_t smem = sizeof(float2) * (size_t(V) * (N + N / 32) + N);
-  auto fn = fft_row_kernel<N, V, INV>;
+  const size_t smem = sizeof(float2) * (size_t(V) * (N + N / 32) + (a.tw_table ? N : 0));
+  auto fn = a.tw_table ? fft_row_kernel<N, V, INV, true> : fft_row_kernel<N, V, INV, false>;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -451,20 +528,29 @@ cudaError_t launch_group_n(const ChannelIO<float> *chans, const int *members, in
 bool fft_rows_supported(int Nu) { return Nu >= 64 && Nu <= 4096 && (Nu & (Nu - 1)) == 0; }
 
 std::vector<float> fft_twiddles(int N) {
+  std::vector<float> t(2 * size_t(N));
+  const double pi = 3.14159265358979323846;
+  for (int m = 0; m < N; ++m) {
+    const double ang = -2.0 * pi * double(m) / double(N);
+    t[2 * size_t(m)] = float(std::cos(ang));
+    t[2 * size_t(m) + 1] = float(std::sin(ang));
+  }
+  return t;
+}
+
+std::vector<float> fft_twiddle_table(int N) {
   std::vector<float> t(2 * size_t(N), 0.f);
   const double pi = 3.14159265358979323846;
   auto radix = [&](int Ns) { return (N / Ns) % 16 == 0 ? 16 : N / Ns; };  // StageRadix
   const int R0 = radix(1);
-  for (int Ns = R0; Ns < N; Ns *= radix(Ns)) {
-    const int R = radix(Ns);
-    for (int r = 1; r < R; ++r)
+  for (int Ns = R0; Ns < N; Ns *= radix(Ns))
+    for (int r = 1; r < radix(Ns); ++r)
       for (int k = 0; k < Ns; ++k) {
-        const double ang = -2.0 * pi * double(r) * double(k) / (double(Ns) * R);
+        const double ang = -2.0 * pi * double(r) * double(k) / (double(Ns) * radix(Ns));
         const size_t e = 2 * (size_t(Ns - R0) + size_t(r - 1) * Ns + k);
         t[e] = float(std::cos(ang));
         t[e + 1] = float(std::sin(ang));
       }
-  }
   return t;
 }
 

@@ -24,14 +24,17 @@ struct FftArgs {
   int Nx = 0, Ny = 0, Nu = 0, Nv = 0, x0 = 0, y0 = 0;
   int ld = 0;                                // row stride of the grid in cells (0: Nu)
   const float *su = nullptr, *sv = nullptr;  // correction per column / row of the image
-  const void *tw_u = nullptr;                // fft_twiddles(Nu)
+  const void *tw_u = nullptr;                // fft_twiddles or fft_twiddle_table of Nu
+  bool tw_table = false;                     // the latter
 };
 
 // True when the fused row passes handle grids Nu wide.
 bool fft_rows_supported(int Nu);
-// The twiddles of an N-point transform's stages, FP64-generated, as interleaved
-// float pairs (N of them, in the layout that fft_kernels.cu names).
+// exp(-2 pi i m / N) for m < N, FP64-generated, as interleaved float pairs.
 std::vector<float> fft_twiddles(int N);
+// Every stage's twiddles (N values, in the layout that fft_kernels.cu names),
+// FP64-generated.
+std::vector<float> fft_twiddle_table(int N);
 // x (Ny x Nx) -> rows y0 ... of grid (Nv x Nu), row-transformed.
 cudaError_t launch_fft_rows_forward(const FftArgs &a, const void *x, void *grid, cudaStream_t s);
 // rows y0 ... of grid (column-transformed) -> x (Ny x Nx).
@@ -48,7 +51,8 @@ struct FftColArgs {
   const void *in = nullptr;
   void *out = nullptr;
   int Nv = 0, W = 0, ld = 0, y0 = 0, Ny = 0;
-  const void *tw_v = nullptr;  // fft_twiddles(Nv)
+  const void *tw_v = nullptr;  // fft_twiddles or fft_twiddle_table of Nv
+  bool tw_table = false;       // the latter
   const void *chans = nullptr;
   const int *members = nullptr;
   int Nu = 0;
@@ -61,7 +65,8 @@ cudaError_t launch_fft_cols(bool inverse, const FftColArgs &c, cudaStream_t s);
 // in one launch (blockIdx.y = member): channel members[k] of the ChannelIO<float>
 // table `chans` reads x_in and writes pad (forward), or reads work and writes
 // x_out (inverse), with its own image size, offsets and corrections; every
-// member's grids have row stride ld.  max_ny is the largest member Ny.
+// member's grids have row stride ld, tw_u is the fft_twiddle_table of Nu, and
+// max_ny is the largest member Ny.
 cudaError_t launch_fft_rows_group(bool inverse, const void *chans, const int *members, int nmembers,
                                   int Nu, int max_ny, int ld, const void *tw_u, cudaStream_t s);
 

@@ -394,13 +394,13 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   cufft_check(cufftPlan2d(&fft_, Nv_, Nu_, Traits<real>::kType), "cufftPlan2d");
   fft_ok_ = true;
   if (sizeof(real) == 4 && fft_rows_supported(Nu_)) {
-    const std::vector<float> twu = fft_twiddles(Nu_);
+    const std::vector<float> twu = strips_ ? fft_twiddle_table(Nu_) : fft_twiddles(Nu_);
     tw_u_.alloc(sizeof(float) * twu.size(), &bytes);
     tw_u_.upload(twu.data(), sizeof(float) * twu.size(), stream_);
     own_cols_ = cfg.fft_columns != 1 && fft_cols_supported(Nv_, Nu_);
     std::vector<float> twv;
     if (own_cols_) {
-      twv = fft_twiddles(Nv_);
+      twv = strips_ ? fft_twiddle_table(Nv_) : fft_twiddles(Nv_);
       tw_v_.alloc(sizeof(float) * twv.size(), &bytes);
       tw_v_.upload(twv.data(), sizeof(float) * twv.size(), stream_);
     } else {
@@ -1037,6 +1037,7 @@ FftArgs OperatorT<real>::fft_args() const {
   f.su = reinterpret_cast<const float *>(su_active());
   f.sv = reinterpret_cast<const float *>(sv_d_.get());
   f.tw_u = tw_u_.get();
+  f.tw_table = strips_;
   return f;
 }
 
@@ -1051,6 +1052,7 @@ FftColArgs OperatorT<real>::col_args(const void *in, void *out) const {
   c.y0 = y0_;
   c.Ny = Ny_;
   c.tw_v = tw_v_.get();
+  c.tw_table = strips_;
   return c;
 }
 
