@@ -172,6 +172,7 @@ cudaError_t launch_grid_group(const ApplyArgs<real> &a, const PolyTable<real> &p
   const size_t smem = grid_smem_bytes(sizeof(real), J, win_rows, win_cols, shape, user,
                                       a.group_cells, poly_nsub(poly));
   ApplyArgs<real> b = a;
+  b.windows = shape.window_count();
   b.win_bytes = int(window_bytes(sizeof(real), win_rows, win_cols, shape, true, a.group_cells));
   return launch_apply<real, true>(false, b, poly, J, ntasks, smem, shape.threads, s);
 }

@@ -41,6 +41,7 @@ struct ApplyArgs {
   int keep_in = 0;
   int64_t slot_stride = 0;          // complex elements per tilebuf slot
   int win_bytes = 0;    // set by the launchers: shared bytes before the batch headers
+  int windows = 0;      // set by the launchers: LaunchShape::window_count()
   // set by the launchers: degrid, the per-warp staging stride; normal, the
   // shared bytes of the grid window before the warp windows
   int stage_bytes = 0;
@@ -59,6 +60,10 @@ constexpr int kNormBlocks = 512;
 
 struct LaunchShape {
   int threads = 128;  // 32 x warps per CTA
+  // G^H and the normal operator: shared-memory windows of a CTA, a divisor of
+  // its warps (0: one per warp).  See FlushOrder in gridding_device.cuh.
+  int windows = 0;
+  int window_count() const { return windows > 0 ? windows : threads / 32; }
 };
 
 // Largest dynamic shared memory a launch of the given shape needs, in bytes:

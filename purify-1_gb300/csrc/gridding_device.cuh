@@ -445,6 +445,34 @@ __global__ void __launch_bounds__(256) degrid_kernel(const ApplyArgs<real> a0,
   cp_async_wait_all();
 }
 
+// Flush order of a CTA with more warps than windows.  Window w takes batches
+// w, w + nwin, w + 2 nwin, ... of the task in that order, as one warp would
+// flush them; warps w, w + nwin, ... (nw / nwin of them) accumulate these
+// batches in turn, each flushing when the warp before it in the list has (a
+// named barrier for each of the nw links, numbers 1 ... nw).  So the windows'
+// sums have the bits that nwin warps give, while the batches of a dense tile
+// are accumulated on more warps.  Every wait is on a batch that its warp
+// flushes unconditionally.
+struct FlushOrder {
+  int link, links, pos, count;  // links: warps of this window; pos: next batch in its list
+  __device__ __forceinline__ FlushOrder(int warp, int nw, int nwin, int nbt) {
+    const int w = warp % nwin;
+    links = nw / nwin;
+    link = 1 + w * links;
+    pos = warp / nwin;
+    count = (nbt - w + nwin - 1) / nwin;
+  }
+  // before and after the flush of batch `pos` of the list
+  __device__ __forceinline__ void wait() const {
+    if (pos > 0)
+      asm volatile("bar.sync %0, 64;" ::"r"(link + (pos - 1) % links) : "memory");
+  }
+  __device__ __forceinline__ void done() {
+    if (pos + 1 < count) asm volatile("bar.arrive %0, 64;" ::"r"(link + pos % links) : "memory");
+    pos += links;
+  }
+};
+
 // Coverage loads the grid kernel keeps in flight per warp (depth, in steps)
 // and how many steps before its gather a caller index is loaded
 // (index_lead).  Wide supports: 2 and 1; a step's arithmetic covers the
@@ -460,8 +488,9 @@ struct GridAhead {
 };
 
 // TAB: stored taps, as in degrid_kernel.
+// ORD: more warps than windows (FlushOrder).
 template <typename real, int J, int G, bool SUB, bool GROUP, bool CALLER = false,
-          bool TAB = false>
+          bool TAB = false, bool ORD = false>
 __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
                                                    const __grid_constant__ PolyTable<real> poly) {
   using C = cplx<real>;
@@ -478,16 +507,17 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
   const int WW = tk.W + JBU - 1, WH = tk.H + JBV - 1, WS = a.win_stride,
             WN = win_cells(WH, WS, G);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nwin = ORD ? a0.windows : nw;
   C *wins = reinterpret_cast<C *>(smem_raw);
   const TaskHeaders th = load_headers(a, tk, smem_raw + a0.win_bytes);
   {
     // zero the warp windows, 16 bytes per store (the windows start 16-byte
     // aligned; an odd FP32 cell count leaves one 8-byte cell at the end)
-    const size_t bytes = size_t(nw) * WN * sizeof(C);
+    const size_t bytes = size_t(nwin) * WN * sizeof(C);
     uint4 *z = reinterpret_cast<uint4 *>(smem_raw);
     for (int idx = threadIdx.x; idx < int(bytes / 16); idx += blockDim.x)
       z[idx] = make_uint4(0u, 0u, 0u, 0u);
-    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nw * WN - 1] = C{0, 0};
+    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nwin * WN - 1] = C{0, 0};
   }
   // tap coefficients of sub-segmented kernels, after the batch headers
   real *csm = reinterpret_cast<real *>(smem_raw + a0.win_bytes + kHeaderBytes);
@@ -496,7 +526,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
   __syncthreads();
   // the visibilities are the previous kernel's output
   pdl_wait();
-  C *mine = wins + warp * WN;
+  C *mine = wins + (ORD ? warp % nwin : warp) * WN;
   const int nbt = tk.batch_end - tk.batch_begin;
   const C *frac = static_cast<const C *>(a.frac);
   const C *vin = static_cast<const C *>(a.slot_in);
@@ -574,6 +604,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
       yq[d] = C{0, 0};
       if (d == 0 || plb < nbt) prefetch(tq[d], yq[d]);
     }
+    FlushOrder turn(warp, nw, nwin, nbt);
     C acc[JBV][JBU];
 #pragma unroll
     for (int jv = 0; jv < JBV; ++jv)
@@ -615,6 +646,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
         code_n = lane_code_at(th, clb + 2 * nw, nbt, lane);
         const int cnt = item_count(code);
         C *blk = mine + win_offset(item_lp(code), item_lq(code), WS, G);
+        if constexpr (ORD) turn.wait();
 #pragma unroll
         for (int jv = 0; jv < JBV; ++jv)
 #pragma unroll
@@ -626,6 +658,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
             acc[jv][ju] = C{0, 0};
             __syncwarp();
           }
+        if constexpr (ORD) turn.done();
       }
       adv(clb, ck);
     }
@@ -637,7 +670,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
   for (int idx = threadIdx.x; idx < WW * WH; idx += blockDim.x, cur.next(WW)) {
     const int e = win_offset(cur.lp, cur.lq, WS, G);
     C s = wins[e];
-    for (int w = 1; w < nw; ++w) {
+    for (int w = 1; w < nwin; ++w) {
       const C o = wins[w * WN + e];
       s.x += o.x;
       s.y += o.y;
@@ -660,7 +693,7 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
 // evaluation per visibility instead of two.  Shared memory: the grid window
 // (a.stage_bytes bytes), the warp windows, then the batch headers at
 // a.win_bytes.
-template <typename real, int J, bool SUB>
+template <typename real, int J, bool SUB, bool ORD>
 __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
                                                      const __grid_constant__ PolyTable<real> poly) {
   using C = cplx<real>;
@@ -671,17 +704,18 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   const Task tk = a.tasks[task_id];
   const int WW = tk.W + J - 1, WH = tk.H + J - 1, WS = a.win_stride, WN = win_cells(WH, WS, G);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nwin = ORD ? a.windows : nw;
   C *gwin = reinterpret_cast<C *>(smem_raw);
   C *wins = reinterpret_cast<C *>(smem_raw + a.stage_bytes);
   const TaskHeaders th = load_headers(a, tk, smem_raw + a.win_bytes);
   {
     // zero the warp windows, 16 bytes per store (stage_bytes is a multiple
     // of 16; an odd FP32 cell count leaves one 8-byte cell at the end)
-    const size_t bytes = size_t(nw) * WN * sizeof(C);
+    const size_t bytes = size_t(nwin) * WN * sizeof(C);
     uint4 *z = reinterpret_cast<uint4 *>(smem_raw + a.stage_bytes);
     for (int idx = threadIdx.x; idx < int(bytes / 16); idx += blockDim.x)
       z[idx] = make_uint4(0u, 0u, 0u, 0u);
-    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nw * WN - 1] = C{0, 0};
+    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nwin * WN - 1] = C{0, 0};
   }
   // tap coefficients of sub-segmented kernels, after the batch headers
   real *csm = reinterpret_cast<real *>(smem_raw + a.win_bytes + kHeaderBytes);
@@ -699,7 +733,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   }
   cp_async_wait_all();
   __syncthreads();
-  C *mine = wins + warp * WN;
+  C *mine = wins + (ORD ? warp % nwin : warp) * WN;
   const int nbt = tk.batch_end - tk.batch_begin;
   const C *frac = static_cast<const C *>(a.frac);
   if (warp < nbt) {
@@ -725,6 +759,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
       t1 = stream_load(frac + slot(plb, pk));
       adv(plb, pk);
     }
+    FlushOrder turn(warp, nw, nwin, nbt);
     C F[J][J], acc[J][J];
     int cnt = 0;
     auto load_block = [&](int code) {
@@ -773,6 +808,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
         code_n = lane_code_at(th, clb + 2 * nw, nbt, lane);
         const int fcnt = item_count(code);
         C *blk = mine + win_offset(item_lp(code), item_lq(code), WS, G);
+        if constexpr (ORD) turn.wait();
 #pragma unroll
         for (int jv = 0; jv < J; ++jv)
 #pragma unroll
@@ -784,6 +820,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
             acc[jv][ju] = C{0, 0};
             __syncwarp();
           }
+        if constexpr (ORD) turn.done();
         adv(clb, ck);
         if (clb < nbt) load_block(code_c);
       } else {
@@ -797,7 +834,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   for (int idx = threadIdx.x; idx < WW * WH; idx += blockDim.x, oc.next(WW)) {
     const int e = win_offset(oc.lp, oc.lq, WS, G);
     C s = wins[e];
-    for (int w = 1; w < nw; ++w) {
+    for (int w = 1; w < nwin; ++w) {
       const C o = wins[w * WN + e];
       s.x += o.x;
       s.y += o.y;
@@ -1150,7 +1187,7 @@ inline int poly_nsub(const PolyTable<real> &poly) {
 inline size_t window_bytes(int precision_bytes, int win_rows, int win_cols, const LaunchShape &shape,
                            bool per_warp, int group = 1) {
   const size_t one = size_t(win_cells(win_rows, win_cols, group)) * 2 * precision_bytes;
-  const size_t b = per_warp ? one * size_t(shape.threads / 32) : one;
+  const size_t b = per_warp ? one * size_t(shape.window_count()) : one;
   return (b + 15) / 16 * 16;
 }
 
@@ -1161,15 +1198,25 @@ template <typename real, int J, int G, bool SUB, bool GROUP>
 cudaError_t launch_one(bool degrid, const ApplyArgs<real> &a, const PolyTable<real> &poly,
                        int ntasks, size_t smem, int threads, cudaStream_t s) {
   auto fn = degrid ? degrid_kernel<real, J, G, SUB, GROUP> : grid_kernel<real, J, G, SUB, GROUP>;
+  const bool ord = !degrid && a.windows * 32 < threads;
+  if constexpr (G == 1 && !GROUP) {
+    if (ord) fn = grid_kernel<real, J, G, SUB, GROUP, false, false, true>;
+  } else if (ord) {
+    return cudaErrorInvalidValue;
+  }
+  if constexpr (sizeof(real) == 4 && J < 6 && G == 1 && !GROUP) {
+    // G^H gathering caller order at narrow supports: deeper prefetch
+    if (!degrid && a.slot_user)
+      fn = ord ? grid_kernel<real, J, G, SUB, GROUP, true, false, true>
+               : grid_kernel<real, J, G, SUB, GROUP, true>;
+  }
   if constexpr (sizeof(real) == 8 && G == 1 && !SUB) {
     // stored taps
     if (a.taps)
       fn = degrid ? degrid_kernel<real, J, G, false, GROUP, true>
                   : grid_kernel<real, J, G, false, GROUP, false, true>;
-  }
-  if constexpr (sizeof(real) == 4 && J < 6 && G == 1 && !GROUP) {
-    // G^H gathering caller order at narrow supports: deeper prefetch
-    if (!degrid && a.slot_user) fn = grid_kernel<real, J, G, SUB, GROUP, true>;
+    if constexpr (!GROUP)
+      if (a.taps && ord) fn = grid_kernel<real, J, G, false, GROUP, false, true, true>;
   }
   if (smem > 48 * 1024) {
     const cudaError_t e =

@@ -46,13 +46,15 @@ namespace {
 // Supports from which the default launch shape and adjoint path change
 // (see the constructor).
 constexpr int kWideSupport = 6;
+// Launch shape of normal_kernel: two windows per CTA (its shared memory holds
+// the grid window besides).
+constexpr LaunchShape kNormalShape{64};
+// Warps that the batches of a task are dealt to, and windows of a G^H CTA: 4
+// below kWideSupport, 2 from there.
+constexpr LaunchShape default_shape(int J) { return LaunchShape{J >= kWideSupport ? 64 : 128}; }
 // Supports from which the adjoint's grid kernel gathers caller order itself
 // by default.
 constexpr int kGatherInGridSupport = 4;
-// Launch shape of normal_kernel: two warps per CTA.  Its two register
-// blocks per lane leave room for few warps, and its shared memory holds the
-// grid window besides the warp windows.
-constexpr LaunchShape kNormalShape{64};
 // Host entry points of FP32 operators: the c128 <-> c64 conversion and the
 // host copies run in up to kCopyChunks chunks of at least kCopyChunkMin
 // values, overlapped (upload_c128, download_c128).
@@ -203,7 +205,9 @@ class OperatorT final : public Operator {
   std::vector<double> su_, sv_;  // 1 / ft kernel at the image pixels (unscaled)
   std::vector<real> su_scaled_, sv_real_;
   PolyTable<real> poly_{};
-  LaunchShape shape_;
+  // CTAs of G, G^H and the normal operator's one pass: the tuning's threads, or
+  // the plan's choice (choose_warps)
+  LaunchShape degrid_shape_, grid_shape_, normal_shape_;
   int ntasks_ = 0, win_rows_ = 0, win_cols_ = 0, win_stride_ = 0, ntu_ = 0, ntv_ = 0;
   int group_ = 1;  // cells per work item along each axis (plan's group)
   int64_t slot_stride_ = 0;
@@ -308,21 +312,14 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   for (int j = 0; j < Ny_; ++j)
     sv_[j] = 1.0 / kern_y.correction((y0_ + j + 0.5) / Nv_ - 0.5);
 
-  // Defaults measured on the 10^7-visibility workload (1024^2 image, KB,
-  // FP32).  Wide supports (J >= 6): 64-thread CTAs, and the adjoint's grid
-  // kernel gathers caller order itself; its per-visibility work hides the
-  // gathers' latency (J = 6: step 0.414 ms; 128 threads 0.423; a separate
-  // gather 0.47).  Narrower supports: 128-thread CTAs.  From J = 4 the grid
-  // kernel gathers caller order with four steps of loads in flight and the
-  // indices three steps ahead (GridAhead; J = 4: adjoint 0.213 ms against
-  // 0.221 with the separate gather, J = 5: 0.233 against 0.241).  Below
-  // J = 4 the steps are too short and the adjoint gathers into slot order
-  // first (J = 2: adjoint 0.209 ms against 0.294).  The forward always
-  // writes caller order directly (scattered stores) unless the tuning asks
-  // for the slot-ordered path.  The w-projection kernels always use the
-  // slot-ordered buffer.
-  const bool wide = J_ >= kWideSupport;
-  shape_.threads = cfg.threads > 0 ? cfg.threads : (wide ? 64 : 128);
+  // The adjoint's grid kernel gathers caller order itself from J = 4: with four
+  // steps of loads in flight and the indices three steps ahead (GridAhead;
+  // 10^7 visibilities, J = 4: adjoint 0.213 ms against 0.221 with the
+  // separate gather, J = 5: 0.233 against 0.241).  Below J = 4 the steps are
+  // too short and the adjoint gathers into slot order first (J = 2: adjoint
+  // 0.209 ms against 0.294).  The forward always writes caller order directly
+  // (scattered stores) unless the tuning asks for the slot-ordered path.  The
+  // band kernels of the row-factor operators use the slot-ordered buffer.
   fused_forward_ = !wmode_ && cfg.fused_permute != 0;
   keep_vis_l2_ = int64_t(sizeof(C)) * M_ <= kKeepVisL2Bytes;
   keep_store_ = cfg.keep_store != 0;
@@ -354,15 +351,16 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
     cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_),
                "cudaDeviceGetAttribute");
     const int nsub = std::max(poly_.nsub_u, poly_.nsub_v);
+    const LaunchShape shape = cfg.threads > 0 ? LaunchShape{cfg.threads} : default_shape(J_);
     const size_t need = std::max(
-        degrid_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, shape_, true, group_, nsub),
-        grid_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, shape_, true, group_, nsub));
+        degrid_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, shape, true, group_, nsub),
+        grid_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, shape, true, group_, nsub));
     if (need > size_t(optin))
       throw Error(kUnsupported, "tile / threads / support need " + std::to_string(need) +
                                     " bytes of shared memory per CTA; the device allows " +
                                     std::to_string(optin));
     const size_t nsm =
-        normal_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, kNormalShape, group_, nsub);
+        normal_smem_bytes(sizeof(real), J_, win_rows_, win_cols_, normal_shape_, group_, nsub);
     const bool want = cfg.normal_pass == 1 || (cfg.normal_pass == 0 && J_ < kWideSupport);
     one_pass_normal_ = want && !split_weights_ && nsm > 0 && nsm <= size_t(optin);
   }
@@ -477,7 +475,7 @@ void OperatorT<real>::init_plain(const OperatorConfig &cfg, int64_t &bytes, Axis
   // 10^7-visibility workload (G^H 224 against 172 us, G 160 against 139).
   rq.group = cfg.cell_group == 0 ? 1 : cfg.cell_group;
   rq.class_cap = cfg.class_cap;
-  rq.warps = shape_.threads / 32;
+  rq.warps = (cfg.threads > 0 ? cfg.threads : default_shape(J_).threads) / 32;
   Plan plan;
   try {
     plan = build_plan(rq);
@@ -485,6 +483,29 @@ void OperatorT<real>::init_plain(const OperatorConfig &cfg, int64_t &bytes, Axis
     throw Error(kInvalidArgument, e.what());
   }
   group_ = plan.group;
+  degrid_shape_.threads = grid_shape_.threads = 32 * rq.warps;
+  normal_shape_ = kNormalShape;
+  if (cfg.threads == 0 && group_ == 1) {
+    // G^H keeps its windows, and with them its bits, whatever its warps
+    // (FlushOrder)
+    int optin = 0;
+    cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_),
+               "cudaDeviceGetAttribute");
+    const int nsub = std::max(poly_.nsub_u, poly_.nsub_v);
+    int most = 8;
+    for (; most > rq.warps; most /= 2) {
+      const LaunchShape s{32 * most};
+      if (std::max(degrid_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols, s, true,
+                                     group_, nsub),
+                   normal_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols, s, group_,
+                                     nsub)) <= size_t(optin))
+        break;
+    }
+    const PlanWarps w = choose_warps(plan, rq.warps, most, sizeof(real));
+    degrid_shape_.threads = 32 * w.degrid;
+    grid_shape_ = LaunchShape{32 * w.grid, rq.warps};
+    normal_shape_.threads = 32 * w.normal;
+  }
   ntasks_ = int(plan.tasks.size());
   win_rows_ = plan.win_rows;
   win_cols_ = plan.win_cols;
@@ -869,7 +890,8 @@ void OperatorT<real>::degrid_slots(const void *grid, void *caller_vis) {
   a.group_cells = group_;
   a.order = task_order_.as<int32_t>();
   mark_begin(kDegrid);
-  cuda_check(launch_degrid<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, shape_, ws_->stream),
+  cuda_check(launch_degrid<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, degrid_shape_,
+                                 ws_->stream),
              "degrid");
   if (split_weights_) {
     if (caller_vis)
@@ -949,7 +971,8 @@ void OperatorT<real>::grid_core(void *grid, const void *vis, const int32_t *slot
   a.order = task_order_.as<int32_t>();
   a.slot_stride = slot_stride_;
   mark_begin(kGrid);
-  cuda_check(launch_grid<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, shape_, ws_->stream),
+  cuda_check(launch_grid<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, grid_shape_,
+                               ws_->stream),
              "grid");
   mark_end(kGrid);
   fold_into(grid, windows, tile_tasks_.as<int32_t>());
@@ -1139,7 +1162,7 @@ void OperatorT<real>::normal_slots(const void *x, void *out) {
     a.order = task_order_.as<int32_t>();
     a.slot_stride = slot_stride_;
     mark_begin(kGrid);
-    cuda_check(launch_normal<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, kNormalShape,
+    cuda_check(launch_normal<real>(a, poly_, J_, ntasks_, win_rows_, win_cols_, normal_shape_,
                                    ws_->stream),
                "normal");
     mark_end(kGrid);

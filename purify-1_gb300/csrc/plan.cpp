@@ -103,6 +103,62 @@ void balance_task_batches(Plan &P, int nw) {
 }
 }  // namespace
 
+// Warps per CTA of the three gridding kernels.  A launch takes about
+//   max(A, B) + alpha min(A, B),
+// A the work of all CTAs over the warps the device holds, every warp of a task
+// counting the task's longest warp and `fixed` (its share of the window to
+// stage, its own to zero and to sum), B the longest warp of the fullest task.
+// More warps shorten B, where a few dense tiles hold most of the
+// visibilities, and lengthen A.  Work is in units of 400 warp instructions;
+// alpha, fixed and the resident warps are fitted to 2, 4 and 8 warps on 30
+// coverages (64^2 to 1024^2 images, 4 x 10^3 to 10^7 visibilities, J = 2 to 8),
+// and a choice other than the default has to win by a margin.  Against the
+// defaults (`dealt`; 2 for the normal operator) G is 1.15, G^H 1.13 and the
+// normal operator 1.32 times as fast on average over these, and none slower.
+// 512^2 image, 2 x 10^6 visibilities, J = 6: G 65 -> 35 us, G^H 131 -> 77;
+// J = 4: G 39 -> 29, G^H 67 -> 50, normal 90 -> 38.  From J = 7 and in FP64 one CTA
+// of 8 warps fills an SM's registers: left out.
+PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) {
+  const size_t nt = P.tasks.size();
+  std::vector<double> cost(nt);
+  for (size_t k = 0; k < nt; ++k) {
+    int64_t c = 0;
+    for (int b = P.tasks[k].batch_begin; b < P.tasks[k].batch_end; ++b)
+      c += kStepCost * P.batch_kmax[b] + kFlushCost;
+    cost[k] = double(c) / 400;
+  }
+  const int J = std::max(P.Ju, P.Jv);
+  if (J >= 7 || precision_bytes == 8) most = std::min(most, 4);
+  auto time = [&](int nw, double fixed, double alpha, double resident) {
+    double all = 0, longest = 0;
+    for (size_t k = 0; k < nt; ++k) {
+      const int n = P.tasks[k].batch_end - P.tasks[k].batch_begin;
+      const double w = cost[k] / std::min(nw, std::max(n, 1)) + fixed;
+      all += nw * w;
+      longest = std::max(longest, w);
+    }
+    all /= resident;
+    return std::max(all, longest) + alpha * std::min(all, longest);
+  };
+  auto pick = [&](int usual, int least, double margin, double fixed, double alpha,
+                  double resident) {
+    const double t0 = time(usual, fixed, alpha, resident);
+    int best = usual;
+    double t = margin * t0;
+    for (int nw = least; nw <= most; nw *= 2)
+      if (nw != usual && time(nw, fixed, alpha, resident) < t) {
+        best = nw;
+        t = time(nw, fixed, alpha, resident);
+      }
+    return best;
+  };
+  PlanWarps w;
+  w.degrid = pick(dealt, 2, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
+  w.grid = pick(dealt, dealt, 0.95, 1, 0, 1500);
+  w.normal = pick(2, 2, 0.95, 8, 0.3, 2500);
+  return w;
+}
+
 Plan build_plan(const PlanRequest &rq) {
   if (rq.M < 0) throw std::invalid_argument("negative number of visibilities");
   if (rq.M > 0 && (!rq.u || !rq.v)) throw std::invalid_argument("u and v must be given");

@@ -46,6 +46,11 @@ struct PlanRequest {
   int warps = 4;
 };
 
+// Warps per CTA of the gridding kernels of one plan.
+struct PlanWarps {
+  int degrid = 4, grid = 4, normal = 2;
+};
+
 // Tiling of one grid axis: tile b covers [start[b], start[b + 1]).
 struct AxisTiling {
   int n = 0;
@@ -106,6 +111,10 @@ PG_HD inline int win_offset(int r, int c, int WS, int group) {
 PG_HD inline int win_cells(int rows, int WS, int group) {
   return rows * WS + (group == 2 ? (rows + 1) / 2 : 0);
 }
+
+// Warps per CTA for the gridding kernels on a plan whose batches are dealt to
+// `dealt` warps or windows; at most `most`.
+PlanWarps choose_warps(const Plan &plan, int dealt, int most, int precision_bytes);
 
 // Builds the plan.  Throws std::invalid_argument on bad input.
 Plan build_plan(const PlanRequest &req);
