@@ -116,8 +116,10 @@ void balance_task_batches(Plan &P, int nw) {
 // defaults (`dealt`; 2 for the normal operator) G is 1.15, G^H 1.13 and the
 // normal operator 1.32 times as fast on average over these, and none slower.
 // 512^2 image, 2 x 10^6 visibilities, J = 6: G 65 -> 35 us, G^H 131 -> 77;
-// J = 4: G 39 -> 29, G^H 67 -> 50, normal 90 -> 38.  From J = 7 and in FP64 one CTA
-// of 8 warps fills an SM's registers: left out.
+// J = 4: G 39 -> 29, G^H 67 -> 50, normal 90 -> 38.  G takes no fewer warps than
+// the default: on tiles of a batch or two they stage the window more slowly
+// (512^2 image, 6,476 visibilities, Phi: 18.5 us with 4, 20.2 with 2).  From
+// J = 7 and in FP64 one CTA of 8 warps fills an SM's registers: left out.
 PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) {
   const size_t nt = P.tasks.size();
   std::vector<double> cost(nt);
@@ -153,7 +155,7 @@ PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) 
     return best;
   };
   PlanWarps w;
-  w.degrid = pick(dealt, 2, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
+  w.degrid = pick(dealt, dealt, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
   w.grid = pick(dealt, dealt, 0.95, 1, 0, 1500);
   w.normal = pick(2, 2, 0.95, 8, 0.3, 2500);
   return w;
