@@ -1008,103 +1008,166 @@ __global__ void __launch_bounds__(128, (sizeof(real) == 4 && J <= 6) ? 4 : 2) wa
   }
 }
 
-// One CTA per tile.  A cell sums, in this order, the windows of its own
-// tile's tasks, then those of the tile above, the tile to the left and the
-// tile above-left, where their J - 1 halo rows / columns reach into it.
-template <typename real>
-__device__ __forceinline__ void fold_tile(const FoldArgs &f, int t) {
-  using C = cplx<real>;
-  // Launched with 32 x 8 threads: a thread owns column lq of a 32-column
-  // chunk and rows ty, ty + 8, ty + 16, ty + 24 of a 32-row chunk, kept in
-  // registers while the task windows are walked (outer loop over tasks).
+// What the fold of one tile reads of the plan: the tile's bounds, its upper and
+// left neighbours' extents and the task ranges of the four tiles.
+struct FoldTile {
+  int P, Q, H, W, Hu, Wl;
+  int own0, own1, up0, up1, lf0, lf1, dg0, dg1;
+};
+__device__ __forceinline__ FoldTile fold_meta(const FoldArgs &f, int t) {
   const int a = t / f.ntu, b = t - a * f.ntu;
   const int a2 = a == 0 ? f.ntv - 1 : a - 1;
   const int b2 = b == 0 ? f.ntu - 1 : b - 1;
   const int tu = a2 * f.ntu + b, tl = a * f.ntu + b2, td = a2 * f.ntu + b2;
-  // independent broadcast loads of the tile's metadata
-  const int P = f.tv_start[a], P1 = f.tv_start[a + 1], Q = f.tu_start[b], Q1 = f.tu_start[b + 1];
-  const int Pu = f.tv_start[a2], Pu1 = f.tv_start[a2 + 1];
-  const int Ql = f.tu_start[b2], Ql1 = f.tu_start[b2 + 1];
-  const int own0 = f.tile_tasks[t], own1 = f.tile_tasks[t + 1];
-  const int up0 = f.tile_tasks[tu], up1 = f.tile_tasks[tu + 1];
-  const int lf0 = f.tile_tasks[tl], lf1 = f.tile_tasks[tl + 1];
-  const int dg0 = f.tile_tasks[td], dg1 = f.tile_tasks[td + 1];
-  const int H = P1 - P, W = Q1 - Q, Hu = Pu1 - Pu, Wl = Ql1 - Ql;
+  // independent broadcast loads
+  FoldTile m;
+  m.P = f.tv_start[a], m.Q = f.tu_start[b];
+  m.H = f.tv_start[a + 1] - m.P, m.W = f.tu_start[b + 1] - m.Q;
+  m.Hu = f.tv_start[a2 + 1] - f.tv_start[a2], m.Wl = f.tu_start[b2 + 1] - f.tu_start[b2];
+  m.own0 = f.tile_tasks[t], m.own1 = f.tile_tasks[t + 1];
+  m.up0 = f.tile_tasks[tu], m.up1 = f.tile_tasks[tu + 1];
+  m.lf0 = f.tile_tasks[tl], m.lf1 = f.tile_tasks[tl + 1];
+  m.dg0 = f.tile_tasks[td], m.dg1 = f.tile_tasks[td + 1];
+  return m;
+}
+
+// One CTA of 32 x kFoldRows threads per tile.  A cell sums, in this order, the
+// windows of its own tile's tasks, then those of the tile above, the tile to
+// the left and the tile above-left, where their J - 1 halo rows / columns
+// reach into it.
+//
+// Bound by load latency: a tile has one task or none in most plans, so a CTA
+// reads one window and some halos and is gone.  What helps is more bytes in
+// flight for each latency of that short life: the first window of each of the
+// four tiles is loaded before any is added (a 0 stands in for one that is not
+// there: a sum that began at +0 keeps its bits), and 128 threads hold 8 cells
+// each in FP32 (4 in FP64, by registers).  Measured with cold caches against 256
+// threads of 4 cells that walked the four tiles one after the other: 31,520
+// tiles of 32^2 201 -> 100 us (4 TB/s), 17,408 of 32^2 101 -> 71, 7,880 of 48^2
+// 142 -> 94; one grid of 63 x 44 mostly ragged tiles 18.4 -> 14.8.
+constexpr int kFoldRows = 4;
+
+// A chunk of 32 columns from c0 and kFoldRows * R rows from r0: thread
+// (lq, ty) owns rows ty + kFoldRows r of column lq, in registers while the
+// task windows are walked.  For halos of at most 8 rows and 32 columns, which
+// then lie in r < 2 of the first chunks.  FULL: the whole chunk is in the tile.
+template <typename real, int R, bool FULL>
+__device__ __forceinline__ void fold_chunk(const FoldArgs &f, const FoldTile &m, int c0, int r0) {
+  using C = cplx<real>;
+  constexpr int T = kFoldRows, U = 8 / T;
+  const int lq = c0 + int(threadIdx.x), lp = r0 + int(threadIdx.y);
+  const int WWo = m.W + f.Ju - 1, WWl = m.Wl + f.Ju - 1;
+  const int64_t ss = f.slot_stride;
+  const C *__restrict__ buf = static_cast<const C *>(f.tilebuf);
+  const bool col = FULL || lq < m.W, left = lq < f.Ju - 1 && col;
+  const C *own = buf + lq + lp * WWo, *up = own + m.Hu * WWo;
+  const C *lf = buf + lq + m.Wl + lp * WWl, *dg = lf + m.Hu * WWl;
+  bool row[R], top[U];
+#pragma unroll
+  for (int r = 0; r < R; ++r) row[r] = FULL || lp + T * r < m.H;
+#pragma unroll
+  for (int r = 0; r < U; ++r) top[r] = lp + T * r < f.Jv - 1 && row[r];
+  C s[R], l0[R], u0[U], d0[U];
+#pragma unroll
+  for (int r = 0; r < R; ++r) s[r] = l0[r] = C{0, 0};
+#pragma unroll
+  for (int r = 0; r < U; ++r) u0[r] = d0[r] = C{0, 0};
+  if (m.own0 < m.own1 && col) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (row[r]) s[r] = own[m.own0 * ss + T * r * WWo];
+  }
+  if (m.up0 < m.up1 && col) {
+#pragma unroll
+    for (int r = 0; r < U; ++r)
+      if (top[r]) u0[r] = up[m.up0 * ss + T * r * WWo];
+  }
+  if (left) {
+    if (m.lf0 < m.lf1) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (row[r]) l0[r] = lf[m.lf0 * ss + T * r * WWl];
+    }
+    if (m.dg0 < m.dg1) {
+#pragma unroll
+      for (int r = 0; r < U; ++r)
+        if (top[r]) d0[r] = dg[m.dg0 * ss + T * r * WWl];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) s[r] = C{real(0) + s[r].x, real(0) + s[r].y};
+  for (int k = m.own0 + 1; k < m.own1; ++k) {
+    C v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = col && row[r] ? own[k * ss + T * r * WWo] : C{0, 0};
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = add2(s[r], v[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < U; ++r) s[r] = add2(s[r], u0[r]);
+  if (col && top[0])
+    for (int k = m.up0 + 1; k < m.up1; ++k) {
+#pragma unroll
+      for (int r = 0; r < U; ++r)
+        if (top[r]) s[r] = add2(s[r], up[k * ss + T * r * WWo]);
+    }
+  if (left) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = add2(s[r], l0[r]);
+    for (int k = m.lf0 + 1; k < m.lf1; ++k) {
+      C v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = row[r] ? lf[k * ss + T * r * WWl] : C{0, 0};
+#pragma unroll
+      for (int r = 0; r < R; ++r) s[r] = add2(s[r], v[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < U; ++r) s[r] = add2(s[r], d0[r]);
+    if (top[0])
+      for (int k = m.dg0 + 1; k < m.dg1; ++k) {
+#pragma unroll
+        for (int r = 0; r < U; ++r)
+          if (top[r]) s[r] = add2(s[r], dg[k * ss + T * r * WWl]);
+      }
+  }
+  const size_t ld = size_t(f.ld ? f.ld : f.Nu);
+  C *g = static_cast<C *>(f.grid) + (size_t(m.P) + lp) * ld + m.Q + lq;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (col && row[r]) g[size_t(T * r) * ld] = s[r];
+}
+
+template <typename real>
+__device__ __forceinline__ void fold_tile(const FoldArgs &f, const FoldTile &m) {
+  using C = cplx<real>;
+  constexpr int R = sizeof(real) == 4 ? 8 : 4, T = kFoldRows;
+  const int P = m.P, Q = m.Q, H = m.H, W = m.W, Hu = m.Hu, Wl = m.Wl;
+  if (f.Jv <= 9 && f.Ju <= 33) {
+    for (int c0 = 0; c0 < W; c0 += 32)
+      for (int r0 = 0; r0 < H; r0 += T * R) {
+        if (W - c0 >= 32 && H - r0 >= T * R)
+          fold_chunk<real, R, true>(f, m, c0, r0);
+        else
+          fold_chunk<real, R, false>(f, m, c0, r0);
+      }
+    return;
+  }
+  const int own0 = m.own0, own1 = m.own1, up0 = m.up0, up1 = m.up1;
+  const int lf0 = m.lf0, lf1 = m.lf1, dg0 = m.dg0, dg1 = m.dg1;
   const int WWo = W + f.Ju - 1, WWl = Wl + f.Ju - 1;
   const int64_t ss = f.slot_stride;
   const C *__restrict__ buf = static_cast<const C *>(f.tilebuf);
   C *__restrict__ grid = static_cast<C *>(f.grid);
-  constexpr int R = 4;
-  if (H == 32 && W == 32 && f.Jv <= 9 && f.Ju <= 33) {
-    // Full tile, halos of at most 8 rows: thread (lq, ty) owns rows ty + 8 r
-    // of column lq; a halo row ty < Jv - 1 is in r = 0 only.  The same sums
-    // in the same order as below, with the per-row tests folded away and two
-    // task windows' loads in flight.
-    const int lq = int(threadIdx.x), ty = int(threadIdx.y);
-    const bool top = ty < f.Jv - 1, left = lq < f.Ju - 1;
-    C s[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) s[r] = C{0, 0};
-    const C *own = buf + lq + ty * WWo;
-#pragma unroll 2
-    for (int k = own0; k < own1; ++k) {
-      const C *w = own + k * ss;
-      C v[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = w[8 * r * WWo];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        s[r].x += v[r].x;
-        s[r].y += v[r].y;
-      }
-    }
-    if (top) {
-      const C *up = buf + Hu * WWo + lq + ty * WWo;
-      for (int k = up0; k < up1; ++k) {
-        const C v = up[k * ss];
-        s[0].x += v.x;
-        s[0].y += v.y;
-      }
-    }
-    if (left) {
-      const C *lf = buf + lq + Wl + ty * WWl;
-#pragma unroll 2
-      for (int k = lf0; k < lf1; ++k) {
-        const C *w = lf + k * ss;
-        C v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = w[8 * r * WWl];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          s[r].x += v[r].x;
-          s[r].y += v[r].y;
-        }
-      }
-      if (top) {
-        const C *dg = buf + Hu * WWl + lq + Wl + ty * WWl;
-        for (int k = dg0; k < dg1; ++k) {
-          const C v = dg[k * ss];
-          s[0].x += v.x;
-          s[0].y += v.y;
-        }
-      }
-    }
-    const size_t ld = size_t(f.ld ? f.ld : f.Nu);
-    C *g = grid + (size_t(P) + ty) * ld + Q + lq;
-#pragma unroll
-    for (int r = 0; r < R; ++r) g[size_t(8 * r) * ld] = s[r];
-    return;
-  }
   for (int c0 = 0; c0 < W; c0 += 32) {
     const int lq = c0 + int(threadIdx.x);
     const bool col = lq < W, left = lq < f.Ju - 1;
-    for (int r0 = 0; r0 < H; r0 += 8 * R) {
+    for (int r0 = 0; r0 < H; r0 += T * R) {
       C s[R];
       int lp[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         s[r] = C{0, 0};
-        lp[r] = r0 + int(threadIdx.y) + 8 * r;
+        lp[r] = r0 + int(threadIdx.y) + T * r;
       }
       // own tile's task windows, in task order
       for (int k = own0; k < own1; ++k) {
