@@ -70,4 +70,19 @@ cudaError_t launch_fft_cols(bool inverse, const FftColArgs &c, cudaStream_t s);
 cudaError_t launch_fft_rows_group(bool inverse, const void *chans, const int *members, int nmembers,
                                   int Nu, int max_ny, int ld, const void *tw_u, cudaStream_t s);
 
+// FP64, power-of-two grids of 64 ... 2048 a side: row and column passes with
+// Z S and S^H Z^H in the row passes.  forward: x -> rows y0 ... of `pad` (the
+// row pass) -> every row of `work`; inverse: `work`, in place, -> x.
+// Unnormalised.  The tables are fft64_twiddle_table of Nu and Nv.
+struct Fft64Args {
+  int Nx = 0, Ny = 0, Nu = 0, Nv = 0, x0 = 0, y0 = 0;
+  const double *su = nullptr, *sv = nullptr;
+  const void *tw_u = nullptr, *tw_v = nullptr;
+};
+bool fft64_supported(int Nu, int Nv);
+std::vector<double> fft64_twiddle_table(int N);
+cudaError_t launch_fft64_forward(const Fft64Args &a, const void *x, void *pad, void *work,
+                                 cudaStream_t s);
+cudaError_t launch_fft64_inverse(const Fft64Args &a, void *work, void *x, cudaStream_t s);
+
 }  // namespace pg

@@ -134,6 +134,7 @@ class OperatorT final : public Operator {
   void grid_on_stream(const void *y, void *grid);
   // Phi' / Phi'^H with visibilities kept in slot order (power method).
   FftArgs fft_args() const;
+  Fft64Args fft64_args() const;
   void forward_slots(const void *x, void *caller_vis = nullptr);
   void adjoint_slots(void *x, const void *caller_vis = nullptr, bool walk = false);
   // G^H of the column-walk plan: ws->slots (walk order) -> task windows -> grid
@@ -219,6 +220,7 @@ class OperatorT final : public Operator {
   // FP32 with a power-of-two grid width: fused row passes + a cuFFT column
   // transform (fft_kernels.h) replace Z S + 2-D FFT and 2-D FFT + S^H Z^H.
   bool fused_fft_ = false;
+  bool fft64_ = false;  // FP64: the passes of fft64_kernels.cu
   cufftHandle fft_cols_ = 0;
   DeviceBuffer tw_u_;
   // own_cols_: the column transforms run as the library's column pass
@@ -406,6 +408,15 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
     }
     cuda_check(cudaStreamSynchronize(stream_), "twiddle upload");
     fused_fft_ = true;
+  }
+  if (sizeof(real) == 8 && cfg.fft_columns != 1 && fft64_supported(Nu_, Nv_)) {
+    const std::vector<double> twu = fft64_twiddle_table(Nu_), twv = fft64_twiddle_table(Nv_);
+    tw_u_.alloc(sizeof(double) * twu.size(), &bytes);
+    tw_u_.upload(twu.data(), sizeof(double) * twu.size(), stream_);
+    tw_v_.alloc(sizeof(double) * twv.size(), &bytes);
+    tw_v_.upload(twv.data(), sizeof(double) * twv.size(), stream_);
+    cuda_check(cudaStreamSynchronize(stream_), "twiddle upload");
+    fft64_ = true;
   }
   cufft_check(cufftSetStream(fft_, stream_), "cufftSetStream");
   size_t ws = 0;
@@ -1065,6 +1076,22 @@ FftArgs OperatorT<real>::fft_args() const {
 }
 
 template <typename real>
+Fft64Args OperatorT<real>::fft64_args() const {
+  Fft64Args f;
+  f.Nx = Nx_;
+  f.Ny = Ny_;
+  f.Nu = Nu_;
+  f.Nv = Nv_;
+  f.x0 = x0_;
+  f.y0 = y0_;
+  f.su = reinterpret_cast<const double *>(su_active());
+  f.sv = reinterpret_cast<const double *>(sv_d_.get());
+  f.tw_u = tw_u_.get();
+  f.tw_v = tw_v_.get();
+  return f;
+}
+
+template <typename real>
 FftColArgs OperatorT<real>::col_args(const void *in, void *out) const {
   FftColArgs c;
   c.in = in;
@@ -1094,6 +1121,12 @@ void OperatorT<real>::forward_grid(const void *x) {
     mark_end(kFftF);
     return;
   }
+  if (fft64_) {
+    mark_begin(kFftF);
+    cuda_check(launch_fft64_forward(fft64_args(), x, ws_->pad, ws_->work, ws_->stream), "fft");
+    mark_end(kFftF);
+    return;
+  }
   mark_begin(kPad);
   cuda_check(launch_pad<real>(x, su_active(), sv_d_.as<real>(), ws_->pad, Nx_, Ny_, Nu_,
                               x0_, y0_, ws_->stream),
@@ -1114,6 +1147,12 @@ void OperatorT<real>::inverse_grid(void *x) {
       cufft_check(Traits<real>::exec(ws_->fft_cols, ws_->work, ws_->work, CUFFT_INVERSE),
                   "cufftExec");
     cuda_check(launch_fft_rows_inverse(fft_args(), ws_->work, x, ws_->stream), "fft rows");
+    mark_end(kFftI);
+    return;
+  }
+  if (fft64_) {
+    mark_begin(kFftI);
+    cuda_check(launch_fft64_inverse(fft64_args(), ws_->work, x, ws_->stream), "fft");
     mark_end(kFftI);
     return;
   }
