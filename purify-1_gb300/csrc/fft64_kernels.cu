@@ -8,9 +8,10 @@
 // Measured on a 1024^2 grid, image 512^2 (us, cold caches): rows 43, columns 74
 // (FP64 pipe 80% busy), against cuFFT's 2-D plan, 88 + 90, with a pad or crop of
 // 5: pair of J = 6 1,204 -> 1,071.
-// A pass lets no dependent launch start early.  The gridding kernels run after
-// it in order of decreasing work, and the CTAs of theirs that came in early
-// would crowd onto the SMs that have room: that pair took 1,177.
+// A pass neither starts before the kernel ahead of it is done nor lets the next
+// one start early.  CTAs that come in early crowd onto the SMs that have room:
+// with both, the pair above took 1,177 us (the gridding kernels run in order of
+// decreasing work), and Phi^H of 2,000 visibilities at 256^2 84 instead of 54.
 // A thread holds one radix-16 butterfly, or as many smaller ones as make 16
 // values, in registers; a CTA holds 16 values a thread in shared memory between
 // stages.
@@ -130,10 +131,9 @@ __device__ __forceinline__ void dft64(double2 *v) {
 // Global loads and stores of the first and last stages: element n of line
 // l0 + l.  Columns: rows y0 ... y0+Ny-1 alone are read (forward; the others
 // are zero) or written (inverse).  Rows: forward reads the image, with the
-// corrections, inverse writes it.  The loads go past L1 (each value is read
-// once): a pass may start before the one before it is done, and the inverse
-// column pass works in place, so a line of the grid that L1 kept as read-only
-// data would be stale for the row pass.
+// corrections, inverse writes it.  The loads go past L1: each value is read
+// once, and the inverse column pass works in place, so nothing may be taken
+// for read-only data.
 template <bool COLS, bool INV>
 __device__ __forceinline__ double2 load64(const Fft64Args &a, const double2 *in,
                                           int line, int n) {
@@ -227,7 +227,6 @@ template <int N, bool COLS, bool INV>
 __global__ void __launch_bounds__(Lines<N, COLS>::T, 512 / Lines<N, COLS>::T)
     fft64_kernel(const Fft64Args a, const double2 *in, double2 *out) {
   extern __shared__ double2 fft64_sm[];
-  dev::pdl_wait();  // `in` is the previous kernel's output
   stage64<N, COLS, INV, 1>(a, in, out, fft64_sm,
                            static_cast<const double2 *>(COLS ? a.tw_v : a.tw_u),
                            int(blockIdx.x) * Lines<N, COLS>::V);
@@ -243,14 +242,14 @@ cudaError_t launch64(const Fft64Args &a, const void *in, void *out, cudaStream_t
     if (e != cudaSuccess) return e;
   }
   const int lines = COLS ? a.Nu : a.Ny;
-  return launch_chain(fn, dim3((lines + L::V - 1) / L::V), dim3(L::T), L::smem, s, a,
-                      static_cast<const double2 *>(in), static_cast<double2 *>(out));
+  fn<<<(lines + L::V - 1) / L::V, L::T, L::smem, s>>>(a, static_cast<const double2 *>(in),
+                                                      static_cast<double2 *>(out));
+  return cudaGetLastError();
 }
 
 template <bool COLS, bool INV>
 cudaError_t launch64_n(const Fft64Args &a, const void *in, void *out, cudaStream_t s) {
   switch (COLS ? a.Nv : a.Nu) {
-    case 64: return launch64<64, COLS, INV>(a, in, out, s);
     case 128: return launch64<128, COLS, INV>(a, in, out, s);
     case 256: return launch64<256, COLS, INV>(a, in, out, s);
     case 512: return launch64<512, COLS, INV>(a, in, out, s);
@@ -262,9 +261,11 @@ cudaError_t launch64_n(const Fft64Args &a, const void *in, void *out, cudaStream
 
 }  // namespace
 
+// Below 128 a pass is a few CTAs' latency: Phi at 64^2 39.2 us, cuFFT's plan 37.2
+// (128^2: 35.1 and 43.3).
 bool fft64_supported(int Nu, int Nv) {
   for (int n : {Nu, Nv})
-    if (n < 64 || n > 2048 || (n & (n - 1)) != 0) return false;
+    if (n < 128 || n > 2048 || (n & (n - 1)) != 0) return false;
   return true;
 }
 

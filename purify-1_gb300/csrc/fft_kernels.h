@@ -70,7 +70,7 @@ cudaError_t launch_fft_cols(bool inverse, const FftColArgs &c, cudaStream_t s);
 cudaError_t launch_fft_rows_group(bool inverse, const void *chans, const int *members, int nmembers,
                                   int Nu, int max_ny, int ld, const void *tw_u, cudaStream_t s);
 
-// FP64, power-of-two grids of 64 ... 2048 a side: row and column passes with
+// FP64, power-of-two grids of 128 ... 2048 a side: row and column passes with
 // Z S and S^H Z^H in the row passes.  forward: x -> rows y0 ... of `pad` (the
 // row pass) -> every row of `work`; inverse: `work`, in place, -> x.
 // Unnormalised.  The tables are fft64_twiddle_table of Nu and Nv.

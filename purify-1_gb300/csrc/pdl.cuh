@@ -32,9 +32,10 @@ __device__ __forceinline__ void pdl_launch_next() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 }  // namespace dev
 
+// launch_chain_if(false, ...) starts the kernel after the previous one is done.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_chain(void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                         cudaStream_t s, Args &&...args) {
+cudaError_t launch_chain_if(bool early, void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t s, Args &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -42,10 +43,16 @@ cudaError_t launch_chain(void (*fn)(KArgs...), dim3 grid, dim3 block, size_t sme
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = kChainPdl ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = kChainPdl && early ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, fn, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_chain(void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t s, Args &&...args) {
+  return launch_chain_if(true, fn, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 }  // namespace pg

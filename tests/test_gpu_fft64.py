@@ -1,4 +1,4 @@
-"""FP64 row and column passes on power-of-two grids of 64 ... 2048 a side: the
+"""FP64 row and column passes on power-of-two grids of 128 ... 2048 a side (a side of 64 takes the plan): the
 operator against the same one on the strided cuFFT plan (fft_columns 1), with
 images that fill their half of the grid, odd ones and single rows or columns.
 
@@ -33,7 +33,8 @@ def test_passes_match_cufft(pg, cuda, ny, nx):
 
 
 @pytest.mark.parametrize("ny,nx,over", [(37, 37, 1.7298), (33, 66, 1.9395), (50, 25, 2.5601),
-                                        (1, 2, 64.0)])
+                                        (1, 2, 64.0), (74, 74, 1.7298),
+                                        (66, 132, 1.9395), (100, 50, 2.5601)])
 def test_odd_images(pg, oracle_mod, cuda, ny, nx, over):
     torch = cuda
     M = 500
