@@ -18,7 +18,7 @@ using namespace dev;
 // channel map[b].x, its block map[b].y, so no block is idle whatever the
 // spread of channel sizes.
 template <typename real>
-__global__ void __launch_bounds__(32 * kFoldRows, sizeof(real) == 4 ? 8 : 4)
+__global__ void __launch_bounds__(32 * FoldShape<real>::rows, sizeof(real) == 4 ? 8 : 4)
     fold_group_kernel(const FoldArgs *__restrict__ folds, const int2 *__restrict__ map) {
   const int2 m = map[blockIdx.x];
   const FoldArgs &f = folds[m.x];
@@ -182,7 +182,7 @@ cudaError_t launch_grid_group(const ApplyArgs<real> &a, const PolyTable<real> &p
 template <typename real>
 cudaError_t launch_fold_group(const FoldArgs *folds, const int2 *map, int nblocks, cudaStream_t s) {
   if (nblocks == 0) return cudaSuccess;
-  fold_group_kernel<real><<<nblocks, dim3(32, kFoldRows), 0, s>>>(folds, map);
+  fold_group_kernel<real><<<nblocks, dim3(32, FoldShape<real>::rows), 0, s>>>(folds, map);
   return cudaGetLastError();
 }
 template <typename real>

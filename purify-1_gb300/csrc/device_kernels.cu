@@ -84,7 +84,7 @@ __global__ void expand_kernel(const cplx<real> *__restrict__ in,
 }
 
 template <typename real>
-__global__ void __launch_bounds__(32 * kFoldRows, sizeof(real) == 4 ? 8 : 4)
+__global__ void __launch_bounds__(32 * FoldShape<real>::rows, sizeof(real) == 4 ? 8 : 4)
     fold_kernel(const FoldArgs f) {
   dev::pdl_launch_next();
   const FoldTile m = fold_meta(f, int(blockIdx.x));  // the plan's, not a kernel's output
@@ -394,7 +394,7 @@ cudaError_t launch_walk_grid(const WalkArgs<real> &a, const PolyTable<real> &pol
 
 template <typename real>
 cudaError_t launch_fold(const FoldArgs &f, cudaStream_t s) {
-  return launch_chain(fold_kernel<real>, dim3(f.ntu * f.ntv), dim3(32, kFoldRows), 0,
+  return launch_chain(fold_kernel<real>, dim3(f.ntu * f.ntv), dim3(32, FoldShape<real>::rows), 0,
                       s, f);
 }
 

@@ -1031,7 +1031,7 @@ __device__ __forceinline__ FoldTile fold_meta(const FoldArgs &f, int t) {
   return m;
 }
 
-// One CTA of 32 x kFoldRows threads per tile.  A cell sums, in this order, the
+// One CTA of 32 x FoldShape::rows threads per tile.  A cell sums, in this order, the
 // windows of its own tile's tasks, then those of the tile above, the tile to
 // the left and the tile above-left, where their J - 1 halo rows / columns
 // reach into it.
@@ -1041,20 +1041,23 @@ __device__ __forceinline__ FoldTile fold_meta(const FoldArgs &f, int t) {
 // flight for each latency of that short life: the first window of each of the
 // four tiles is loaded before any is added (a 0 stands in for one that is not
 // there: a sum that began at +0 keeps its bits), and 128 threads hold 8 cells
-// each in FP32 (4 in FP64, by registers).  Measured with cold caches against 256
+// each in FP32 (FP64: 256 threads of 2 cells, by registers).  Measured with cold caches against 256
 // threads of 4 cells that walked the four tiles one after the other: 31,520
 // tiles of 32^2 201 -> 100 us (4 TB/s), 17,408 of 32^2 101 -> 71, 7,880 of 48^2
 // 142 -> 94; one grid of 63 x 44 mostly ragged tiles 18.4 -> 14.8.
-constexpr int kFoldRows = 4;
+template <typename real>
+struct FoldShape {
+  static constexpr int rows = sizeof(real) == 4 ? 4 : 8, cells = sizeof(real) == 4 ? 8 : 2;
+};
 
-// A chunk of 32 columns from c0 and kFoldRows * R rows from r0: thread
-// (lq, ty) owns rows ty + kFoldRows r of column lq, in registers while the
+// A chunk of 32 columns from c0 and T * R rows from r0: thread (lq, ty) owns
+// rows ty + T r of column lq, in registers while the
 // task windows are walked.  For halos of at most 8 rows and 32 columns, which
 // then lie in r < 2 of the first chunks.  FULL: the whole chunk is in the tile.
 template <typename real, int R, bool FULL>
 __device__ __forceinline__ void fold_chunk(const FoldArgs &f, const FoldTile &m, int c0, int r0) {
   using C = cplx<real>;
-  constexpr int T = kFoldRows, U = 8 / T;
+  constexpr int T = FoldShape<real>::rows, U = 8 / T;
   const int lq = c0 + int(threadIdx.x), lp = r0 + int(threadIdx.y);
   const int WWo = m.W + f.Ju - 1, WWl = m.Wl + f.Ju - 1;
   const int64_t ss = f.slot_stride;
@@ -1140,7 +1143,7 @@ __device__ __forceinline__ void fold_chunk(const FoldArgs &f, const FoldTile &m,
 template <typename real>
 __device__ __forceinline__ void fold_tile(const FoldArgs &f, const FoldTile &m) {
   using C = cplx<real>;
-  constexpr int R = sizeof(real) == 4 ? 8 : 4, T = kFoldRows;
+  constexpr int R = FoldShape<real>::cells, T = FoldShape<real>::rows;
   const int P = m.P, Q = m.Q, H = m.H, W = m.W, Hu = m.Hu, Wl = m.Wl;
   if (f.Jv <= 9 && f.Ju <= 33) {
     for (int c0 = 0; c0 < W; c0 += 32)
