@@ -542,7 +542,8 @@ void OperatorT<real>::init_plain(const OperatorConfig &cfg, int64_t &bytes, Axis
   if constexpr (sizeof(real) == 8) {
     // Stored taps, 16 J bytes per slot.  Measured on a 512^2 image with
     // 2 x 10^6 visibilities, J = 6: Phi then Phi^H 3142 us with the
-    // polynomials, 1700 with the table (192 MB).
+    // polynomials, 1700 with the table (192 MB; 1070 with the FP64 FFT
+    // passes and the launch shapes of today).
     const size_t tb = sizeof(real) * 2 * size_t(J_) * size_t(S_);
     size_t free_b = 0, total_b = 0;
     cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
