@@ -540,8 +540,8 @@ __global__ void __launch_bounds__(kDegridWarps * 32, 14 / kDegridWarps) wstrip_d
   const float2 *grid = static_cast<const float2 *>(a.grid);
   float2 *out = static_cast<float2 *>(a.vis_out);
   // block column b of the task (columns Q + 8 b ...), rows and columns
-  // wrapped; two cells at a time where the rows are 16-byte aligned
-  const bool wide = a.Nu % 2 == 0;
+  // wrapped; two cells at a time where every row is 16-byte aligned
+  const bool wide = a.wide;
   auto load_block = [&](int b, int place) {
     if (wide) {
       const int c = 2 * (threadIdx.x & 3);
@@ -799,7 +799,10 @@ cudaError_t launch_tiles(bool degrid, const WStripArgs &a, cudaStream_t s) {
 }  // namespace
 
 cudaError_t launch_wstrip_degrid(const WStripArgs &a, cudaStream_t s) {
-  return launch_tiles(true, a, s);
+  WStripArgs b = a;
+  // a caller's grid need only be aligned as complex<float> is
+  b.wide = a.Nu % 2 == 0 && reinterpret_cast<uintptr_t>(a.grid) % 16 == 0;
+  return launch_tiles(true, b, s);
 }
 cudaError_t launch_wstrip_grid(const WStripArgs &a, cudaStream_t s) {
   return launch_tiles(false, a, s);

@@ -136,3 +136,34 @@ def test_non_finite_values_stay_in_their_footprint(pg, cuda):
     f0, f1 = vis0.cpu().numpy(), vis1.cpu().numpy()
     assert not np.isfinite(f1[hit]).any() and np.isfinite(f1[~hit]).all()
     assert rel_l2(f1[~hit], f0[~hit]) < TOL
+
+
+@pytest.mark.parametrize("w_rows", [True, False])
+def test_grids_and_visibilities_of_any_alignment(pg, cuda, w_rows):
+    """G and G^H on views one element into their buffers (8 bytes past a
+    16-byte boundary): the same values are copied, so the bits are those of
+    aligned buffers."""
+    torch = cuda
+    n, M = 48, 700
+    N = 2 * n
+    rng = np.random.default_rng(21)
+    u, v = rng.uniform(-n, n, M), rng.uniform(-n, n, M)
+    kw = (dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=9) if w_rows else
+          dict(kernel="kb", Ju=12, Jv=12))
+    op = pg.MeasurementOperator(u, v, _w(rng, M, N) if w_rows else None, None, n, n, 2.0,
+                                power_iters=0, precision="fp32", **kw)
+    z = torch.from_numpy(rng.standard_normal(2 * (N * N + M))).float().cuda()
+    out = []
+    for shift in (0, 1):
+        def buf(size):
+            t = torch.zeros(size + 2, dtype=torch.complex64, device="cuda")[shift:shift + size]
+            assert t.data_ptr() % 16 == 8 * shift
+            return t
+        g, y = buf(N * N), buf(M)
+        g.copy_(torch.view_as_complex(z[:2 * N * N].view(-1, 2)))
+        y.copy_(torch.view_as_complex(z[2 * N * N:].view(-1, 2)))
+        vis, grid = buf(M), buf(N * N)
+        op.degrid_into(g, vis)
+        op.grid_into(y, grid)
+        out.append((vis, grid))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
