@@ -237,6 +237,7 @@ bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
   WStripPlan W;
   const int64_t M = plan.M;
   W.tiles = (plan.Smax + 7 + 7) / 8;
+  if (W.tiles > kMaxStripTiles) return false;
   W.rows = plan.Smax + kStripRows - 1;
   W.strips = (plan.Nv + kStripRows - 1) / kStripRows;
   W.cols = (plan.Nu + kStripCols - 1) / kStripCols;

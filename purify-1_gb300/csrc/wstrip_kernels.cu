@@ -4,25 +4,35 @@
 // A row K = sum_e A_e B_e^T touches S x S cells, so a run of rows whose
 // footprints start in the same 8 x 8 cells is a matrix product over a few
 // 8 x 8 blocks of the grid.  Both kernels give a warp such runs and use
-// mma.m16n8k8 with TF32 operands: the 16 rows are the real and the imaginary
-// parts of 8 values, multiplied by the real parts of the other operand and,
-// in a second product, by its imaginary parts.
+// mma.m16n8k16 with BF16 operands: the 16 rows are the real and the imaginary
+// parts of 8 values, the columns the real and the imaginary parts of 8 terms.
 //
-// Precision.  Every operand x is split into hi + lo with hi = x rounded to 11
-// bits; lo is then exact in 12 bits and TF32 keeps 11 of them.  The products
-// hi hi, hi lo and lo hi are summed, which leaves about 2^-24 of a product.
-// The unit truncates its sums, so each product starts from zero and is added
-// to the FP32 sums outside with rounding.
+// Precision.  Every operand x is split into three pieces of 8 bits, x = x1 + x2 +
+// x3, each the BF16 nearest to what the ones before it leave (a split of FP32
+// into narrower pieces whose products are summed in FP32: Markidis et al. 2018,
+// Ootomo and Yokota 2022).  The split is exact, 24 bits in all.  Six of the nine
+// products are summed, the smallest first:
+//   a3 b1, a1 b3, a2 b2, a1 b2, a2 b1, a1 b1;
+// what is left out (a2 b3, a3 b2, a3 b3) is below 2^-24 of a product, 2^-27 in the
+// mean.  The 16 columns of an instruction hold both halves of a complex product:
+// 8 terms times real parts, 8 times imaginary parts.  The unit truncates its
+// sums, so each block's product starts from zero and is added to the FP32 sums
+// outside with rounding.
 //
-// What bounds them: on paper the mma rate, measured 0.51 m16n8k8 per cycle and
-// SM for TF32.  A 1024^2 image with 2 x 10^6 rows of 4 to 24 taps needs 15.8 M
-// of them per direction, 108 us; G takes 308 us and G^H 313 (0.496 and 0.936 ms
-// with the band kernels of wkernels.cu), at 40% of the issue slots: the
-// registers of the blocks and shared memory leave 12 to 14 warps an SM, whose
-// chains of dependent products and splits are then the limit.
+// Error of G and of G^H alone, random values, 10^6 rows of 4 to 24 taps (relative L2
+// against FP64): 7.7e-8 and 1.16e-7; the band kernels of wkernels.cu 8.3e-8 and
+// 1.66e-7.
+//
+// What bounds them: on paper the mma rate, measured 0.5 a cycle and SM.  A 1024^2
+// image with 10^6 rows of 4 to 24 taps takes 210 us (G) and 280 (G^H), 269 and 542
+// with the band kernels, 187 and 261 with two TF32 pieces of 11 bits, which lost
+// precision (1.0e-7 in G).  The registers of the blocks and shared memory leave
+// 10 to 14 warps an SM, whose chains of dependent products and splits are the
+// limit.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "cplx_ops.cuh"
 #include "pdl.cuh"
@@ -37,39 +47,101 @@ using dev::fma2;
 // Warps of a G^H CTA; they share nothing but the shared-memory array.
 constexpr int kStripWarps = 2;
 
-struct Tf32 {
-  uint32_t hi, lo;
+// The three pieces of two values, the first in the lower halves: two columns of
+// an operand, so that the terms t and t + 4 of a lane are columns 2 t and 2 t + 1.
+struct Pieces {
+  uint32_t p[3];
 };
-__device__ __forceinline__ Tf32 split(float x) {
-  Tf32 r;
-  r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  r.lo = __float_as_uint(x - __uint_as_float(r.hi));
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
   return r;
 }
-// x (1 + kTrunc): one operand of each product makes up for what the unit's
-// truncation takes from a product on average (measured 4.0e-8 of it over
-// random operands, whatever the number of terms).  The unit reads the upper
-// 19 bits of an operand; lo is rounded to them here.
-constexpr float kTrunc = 4.0e-8f;
-__device__ __forceinline__ Tf32 split_up(float x) {
-  Tf32 r;
-  r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  r.lo = __float_as_uint(fmaf(x, kTrunc, x - __uint_as_float(r.hi))) + 0x1000u;
-  return r;
+// Two complex values: the pieces of their real and of their imaginary parts.
+struct Split {
+  Pieces re, im;
+};
+// what the pieces p leave of the values
+__device__ __forceinline__ void split_rest(float2 &v0, float2 &v1, uint32_t re, uint32_t im) {
+  const float2 minus = make_float2(-1.f, -1.f);
+  v0 = fma2(make_float2(__uint_as_float(re << 16), __uint_as_float(im << 16)), minus, v0);
+  v1 = fma2(make_float2(__uint_as_float(re & 0xffff0000u), __uint_as_float(im & 0xffff0000u)),
+            minus, v1);
+}
+template <bool UP>
+__device__ __forceinline__ Split split(float2 v0, float2 v1) {
+  // x (1 + kTrunc): one operand of each product makes up for what the unit's
+  // truncation takes from a product on average (measured 3.5 to 4.0e-8 of it:
+  // random, same-sign and nearly equal operands, 1 to 8 terms).
+  constexpr float kTrunc = 4.0e-8f;
+  const float2 x0 = v0, x1 = v1;
+  Split s;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s.re.p[k] = pack_bf16(v0.x, v1.x);
+    s.im.p[k] = pack_bf16(v0.y, v1.y);
+    if (k < 2) split_rest(v0, v1, s.re.p[k], s.im.p[k]);
+    if (UP && k == 0) {
+      v0 = fma2(x0, make_float2(kTrunc, kTrunc), v0);
+      v1 = fma2(x1, make_float2(kTrunc, kTrunc), v1);
+    }
+  }
+  return s;
 }
 
-// d = a b (16 x 8 by 8 x 8), and d += a b
-__device__ __forceinline__ void mma0(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+// d = a b (16 x 16 by 16 x 8), and d += a b
+__device__ __forceinline__ void mma0(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                     uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
       "{%8, %9}, {%10, %10, %10, %10};"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                    uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
       "{%8, %9}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The left operand: rows g and g + 8 at the columns of the real parts, rows g
+// and g + 8 at those of the imaginary parts.
+struct Rows {
+  uint32_t p[3][4];
+};
+__device__ __forceinline__ Rows rows(const Pieces &re0, const Pieces &im0, const Pieces &re1,
+                                     const Pieces &im1) {
+  Rows r;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.p[k][0] = re0.p[k];
+    r.p[k][1] = im0.p[k];
+    r.p[k][2] = re1.p[k];
+    r.p[k][3] = im1.p[k];
+  }
+  return r;
+}
+__device__ __forceinline__ Pieces negate(Pieces x) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) x.p[k] ^= 0x80008000u;
+  return x;
+}
+// d = left operand times right operand for TV blocks, independent chains of
+// six products: of the blocks i, left operand a(i) and right operand b(i).
+template <int TV, typename A, typename B>
+__device__ __forceinline__ void multiply(float (&d)[TV][4], A a, B b) {
+  constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {0, 1}, {1, 0}, {0, 0}};
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+#pragma unroll
+    for (int i = 0; i < TV; ++i) {
+      const uint32_t(&l)[4] = a(i).p[order[k][0]];
+      const uint32_t re = b(i).re.p[order[k][1]], im = b(i).im.p[order[k][1]];
+      if (k == 0)
+        mma0(d[i], l[0], l[1], l[2], l[3], re, im);
+      else
+        mma(d[i], l[0], l[1], l[2], l[3], re, im);
+    }
 }
 // One factor pair (WTerm) as a lane needs it.
 struct Term {
@@ -134,84 +206,87 @@ __device__ __forceinline__ unsigned smem_address(const void *p) {
 // Eight terms of G^H: lane (g, t) holds A of the terms t and t + 4 at the rows
 // 8 i + g, times conj(weight) y, and B of the same terms at the columns
 // 8 j + g.  Adds scale conj(A) conj(B) z to TV x tu window blocks from block
-// row H on: with conj(A) z = r + i s, the products with B's real parts give
-// (r + i s) B.x, those with its imaginary parts (r + i s) B.y, of which -i
-// times is added.  The blocks of a column are independent chains.
+// row H on: with conj(A) z = r + i s, (r + i s) (B.x - i B.y) is the product of
+// the rows (r, s) with B's real parts and (s, -r) with its imaginary parts.  The
+// blocks of a column are independent chains.
 template <int H, int TV, int TM>
-__device__ __forceinline__ void grid_oct_rows(float2 (&acc)[TM + 1][TM][2],
-                                              const float4 (*A)[32], const float4 (*B)[32],
-                                              float2 z0, float2 z1, float scale, int tu) {
-  uint32_t ah[TV][4], al[TV][4];
+__device__ __forceinline__ void grid_column(float2 (&acc)[TM + 1][TM][2], const Rows (&a)[TM],
+                                            const Split &b, float scale, int j) {
+  float c[TV][4];
+  multiply<TV>(c, [&](int i) -> const Rows & { return a[i]; },
+               [&](int) -> const Split & { return b; });
 #pragma unroll
-  for (int i = 0; i < TV; ++i) {
-    const float4 v = A[i][0];
-    const float x[4] = {fmaf(v.x, z0.x, v.y * z0.y), fmaf(v.x, z0.y, -(v.y * z0.x)),
-                        fmaf(v.z, z1.x, v.w * z1.y), fmaf(v.z, z1.y, -(v.w * z1.x))};
+  for (int i = 0; i < TV; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const Tf32 p = split(x[e]);
-      ah[i][e] = p.hi;
-      al[i][e] = p.lo;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < TM; ++j)
-    if (j < tu) {
-      const float4 v = B[j][0];
-      const float part[2][2] = {{v.x, v.z}, {v.y, v.w}};
-      // both parts together where the rows alone are too few chains
-      constexpr int PARTS = TV <= 2 ? 2 : 1;
-#pragma unroll
-      for (int im0 = 0; im0 < 2; im0 += PARTS) {
-        uint32_t bh[PARTS][2], bl[PARTS][2];
-        float c[PARTS][TV][4];
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k) {
-          const Tf32 p = split_up(part[im0 + k][0]), q = split_up(part[im0 + k][1]);
-          bh[k][0] = p.hi;
-          bh[k][1] = q.hi;
-          bl[k][0] = p.lo;
-          bl[k][1] = q.lo;
-        }
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) mma0(c[k][i], al[i], bh[k]);
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) mma(c[k][i], ah[i], bl[k]);
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) mma(c[k][i], ah[i], bh[k]);
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) {
-            const int im = im0 + k;
-            float2(&d)[2] = acc[H + i][j];
-            const float2 re = make_float2(c[k][i][0], c[k][i][1]), m = make_float2(c[k][i][2], c[k][i][3]);
-            const float2 plus = make_float2(scale, scale), minus = make_float2(-scale, -scale);
-            d[im] = fma2(re, im ? minus : plus, d[im]);
-            d[1 - im] = fma2(m, plus, d[1 - im]);
-          }
-      }
-    }
+    for (int h = 0; h < 2; ++h)
+      acc[H + i][j][h] = fma2(make_float2(c[i][2 * h], c[i][2 * h + 1]), make_float2(scale, scale),
+                              acc[H + i][j][h]);
 }
-template <int H, int TM>
+template <int N>
+using Int = std::integral_constant<int, N>;
+// Calls f(Int<H>, Int<TV>) for the shape of an octet.
+template <int H, int TM, typename F>
+__device__ __forceinline__ void with_shape(int tv, F f) {
+  if constexpr (TM >= 4)
+    if (tv == 4) return f(Int<H>(), Int<4>());
+  if constexpr (TM >= 3)
+    if (tv == 3) return f(Int<H>(), Int<3>());
+  if constexpr (TM >= 2)
+    if (tv == 2) return f(Int<H>(), Int<2>());
+  f(Int<H>(), Int<1>());
+}
+// At TM = 4 the columns are outside and the shape is looked at for each: with
+// every shape's columns unrolled, splits and all, the code outgrows the
+// instruction cache (warps of one SM are in different shapes).
+template <int TM>
 __device__ __forceinline__ void grid_oct(float2 (&acc)[TM + 1][TM][2], const float4 (*A)[32],
                                          const float4 (*B)[32], float2 z0, float2 z1, float scale,
-                                         int tv, int tu) {
-  if constexpr (TM >= 5)
-    if (tv == 5) return grid_oct_rows<H, 5, TM>(acc, A, B, z0, z1, scale, tu);
-  if constexpr (TM >= 4)
-    if (tv == 4) return grid_oct_rows<H, 4, TM>(acc, A, B, z0, z1, scale, tu);
-  if constexpr (TM >= 3)
-    if (tv == 3) return grid_oct_rows<H, 3, TM>(acc, A, B, z0, z1, scale, tu);
-  if constexpr (TM >= 2)
-    if (tv == 2) return grid_oct_rows<H, 2, TM>(acc, A, B, z0, z1, scale, tu);
-  grid_oct_rows<H, 1, TM>(acc, A, B, z0, z1, scale, tu);
+                                         bool half, int tv, int tu) {
+  Rows a[TM];
+  auto split_column = [&](int j) {
+    const float4 v = B[j][0];
+    return split<true>(make_float2(v.x, v.y), make_float2(v.z, v.w));
+  };
+  auto split_rows = [&](int i) {
+    const float4 v = A[i][0];
+    const Split x = split<false>(
+        make_float2(fmaf(v.x, z0.x, v.y * z0.y), fmaf(v.x, z0.y, -(v.y * z0.x))),
+        make_float2(fmaf(v.z, z1.x, v.w * z1.y), fmaf(v.z, z1.y, -(v.w * z1.x))));
+    a[i] = rows(x.re, x.im, x.im, negate(x.re));
+  };
+  if constexpr (TM >= 4) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+      if (i < tv) split_rows(i);
+#pragma unroll
+    for (int j = 0; j < TM; ++j)
+      if (j < tu) {
+        const Split b = split_column(j);
+        auto column = [&](auto h, auto n) {
+          grid_column<decltype(h)::value, decltype(n)::value, TM>(acc, a, b, scale, j);
+        };
+        if (half)
+          with_shape<1, TM>(tv, column);
+        else
+          with_shape<0, TM>(tv, column);
+      }
+  } else {
+    auto columns = [&](auto h, auto n) {
+      constexpr int H = decltype(h)::value, TV = decltype(n)::value;
+#pragma unroll
+      for (int i = 0; i < TV; ++i) split_rows(i);
+#pragma unroll
+      for (int j = 0; j < TM; ++j)
+        if (j < tu) {
+          const Split b = split_column(j);
+          grid_column<H, TV, TM>(acc, a, b, scale, j);
+        }
+    };
+    if (half)
+      with_shape<1, TM>(tv, columns);
+    else
+      with_shape<0, TM>(tv, columns);
+  }
 }
 
 // The same eight terms cell by cell: only cells of a term's footprint are
@@ -280,7 +355,7 @@ struct GridShared {
   int4 terms[4][2 * kOctTerms];
 };
 template <int TM>
-__global__ void __launch_bounds__(kStripWarps * 32, TM == 5 ? 4 : 5) wstrip_grid_kernel(const WStripArgs a) {
+__global__ void __launch_bounds__(kStripWarps * 32, 5) wstrip_grid_kernel(const WStripArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   dev::pdl_launch_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -394,10 +469,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, TM == 5 ? 4 : 5) wstrip_grid
       }
       const float4(*sa)[32] = reinterpret_cast<const float4(*)[32]>(&st.A[0][lane]);
       const float4(*sb)[32] = reinterpret_cast<const float4(*)[32]>(&st.B[0][lane]);
-      if ((blocks >> 8) & 1)
-        grid_oct<1, TM>(acc, sa, sb, z0, z1, scale, tv, tu);
-      else
-        grid_oct<0, TM>(acc, sa, sb, z0, z1, scale, tv, tu);
+      grid_oct<TM>(acc, sa, sb, z0, z1, scale, (blocks >> 8) & 1, tv, tu);
       issue(st);
     }
     oe = oe1;
@@ -448,64 +520,30 @@ template <int TV, int TM>
 __device__ __forceinline__ void degrid_oct_rows(float2 (&T)[TM][2], const float4 (*B)[32],
                                                 const float2 (*ring)[8 * (TM + 1) * 8], int base,
                                                 int row0, int tu, int g, int t) {
+  // not unrolled: with every shape's columns unrolled the code outgrows the
+  // instruction cache
+#pragma unroll 1
+  for (int j = 0; j < tu; ++j) {
+    int place = base + j;
+    if (place >= TM + 1) place -= TM + 1;
+    const float2 *blk = ring[place] + block_at(row0 + g, t);  // block_at(row + 8, c): 64 further
+    const int other = block_at(g, t + 4) - block_at(g, t);
+    const float4 v = B[j][0];
+    const Split f = split<true>(make_float2(v.x, v.y), make_float2(v.z, v.w));
+    // (bx + i by) (gr + i gi): the rows (bx, by) times gr, (-by, bx) times gi
+    const Rows a = rows(f.re, f.im, negate(f.im), f.re);
+    Split grid[TV];
 #pragma unroll
-  for (int j = 0; j < TM; ++j)
-    if (j < tu) {
-      int place = base + j;
-      if (place >= TM + 1) place -= TM + 1;
-      const float2 *blk = ring[place] + block_at(row0 + g, t);  // block_at(row + 8, c): 64 further
-      const int other = block_at(g, t + 4) - block_at(g, t);
-      const float4 v = B[j][0];
-      const float x[4] = {v.x, v.y, v.z, v.w};
-      uint32_t ah[4], al[4];
+    for (int i = 0; i < TV; ++i) grid[i] = split<false>(blk[64 * i], blk[64 * i + other]);
+    float c[TV][4];
+    multiply<TV>(c, [&](int) -> const Rows & { return a; },
+                 [&](int i) -> const Split & { return grid[i]; });
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const Tf32 p = split_up(x[e]);
-        ah[e] = p.hi;
-        al[e] = p.lo;
-      }
-      float2 g0[TV], g1[TV];
+    for (int i = 0; i < TV; ++i)
 #pragma unroll
-      for (int i = 0; i < TV; ++i) {
-        g0[i] = blk[64 * i];
-        g1[i] = blk[64 * i + other];
-      }
-      constexpr int PARTS = TV <= 2 ? 2 : 1;
-#pragma unroll
-      for (int im0 = 0; im0 < 2; im0 += PARTS) {
-        uint32_t bh[PARTS][TV][2], bl[PARTS][TV][2];
-        float c[PARTS][TV][4];
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) {
-            const Tf32 p = split(im0 + k ? g0[i].y : g0[i].x), q = split(im0 + k ? g1[i].y : g1[i].x);
-            bh[k][i][0] = p.hi;
-            bh[k][i][1] = q.hi;
-            bl[k][i][0] = p.lo;
-            bl[k][i][1] = q.lo;
-            mma0(c[k][i], al, bh[k][i]);
-          }
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) mma(c[k][i], ah, bl[k][i]);
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) mma(c[k][i], ah, bh[k][i]);
-#pragma unroll
-        for (int k = 0; k < PARTS; ++k)
-#pragma unroll
-          for (int i = 0; i < TV; ++i) {
-            // (bx + i by) gr, and i times (bx + i by) gi
-            const int im = im0 + k;
-            const float2 re = make_float2(c[k][i][0], c[k][i][1]), m = make_float2(c[k][i][2], c[k][i][3]);
-            T[i][im] = add2(T[i][im], re);
-            T[i][1 - im] = im ? fma2(m, make_float2(-1.f, -1.f), T[i][0]) : add2(T[i][1], m);
-          }
-      }
-    }
+      for (int h = 0; h < 2; ++h)
+        T[i][h] = add2(T[i][h], make_float2(c[i][2 * h], c[i][2 * h + 1]));
+  }
 }
 
 // G, kDegridWarps warps per task.  The grid blocks over the current group and
@@ -631,8 +669,6 @@ __global__ void __launch_bounds__(kDegridWarps * 32, 14 / kDegridWarps) wstrip_d
       for (int i = 0; i < TM; ++i) T[i][0] = T[i][1] = make_float2(0.f, 0.f);
       const float2(*rg)[ROWS * 8] = ring;
       bool todo = true;
-      if constexpr (TM >= 5)
-        if (tv == 5) degrid_oct_rows<5, TM>(T, B, rg, base, row0, tu, g, t), todo = false;
       if constexpr (TM >= 4)
         if (tv == 4) degrid_oct_rows<4, TM>(T, B, rg, base, row0, tu, g, t), todo = false;
       if constexpr (TM >= 3)
@@ -791,7 +827,6 @@ cudaError_t launch_tiles(bool degrid, const WStripArgs &a, cudaStream_t s) {
     case 2: return launch_strip<2>(degrid, a, s);
     case 3: return launch_strip<3>(degrid, a, s);
     case 4: return launch_strip<4>(degrid, a, s);
-    case 5: return launch_strip<5>(degrid, a, s);
   }
   return cudaErrorInvalidValue;
 }

@@ -34,9 +34,6 @@ struct WStripFoldArgs {
 
 // Values of slack before and after the factors (WStripArgs::factors).
 constexpr int kStripSlack = 64;
-// Largest WStripPlan::tiles the kernels are built for (support 32).
-constexpr int kMaxStripTiles = 5;
-
 cudaError_t launch_wstrip_degrid(const WStripArgs &a, cudaStream_t s);
 cudaError_t launch_wstrip_grid(const WStripArgs &a, cudaStream_t s);
 cudaError_t launch_wstrip_fold(const WStripFoldArgs &f, cudaStream_t s);

@@ -1,10 +1,9 @@
 """The tensor-core row kernels (FP32 w-projection rows, supports of 9 to 32
 taps, Ju != Jv) at the edges of their blocks, against the FP64 oracle.
 
-Tolerance (relative L2): 2e-6.  Operands are split so that a product keeps
-about 2^-23 of itself; with sums of a few hundred terms of random sign the
-result is within a few times that, 5e-7, and a lost or misplaced tap would
-show at 1e-3.  Non-finite values stay inside the footprints they belong to;
+Tolerance (relative L2): 2e-6.  A product keeps about 2^-24 of itself; with
+sums of a few hundred terms of random sign the result is within a few times
+that, 5e-7, and a lost or misplaced tap would show at 1e-3.  Non-finite values stay inside the footprints they belong to;
 the finite rest is held to the same tolerance."""
 import numpy as np
 import pytest
@@ -167,3 +166,38 @@ def test_grids_and_visibilities_of_any_alignment(pg, cuda, w_rows):
         op.grid_into(y, grid)
         out.append((vis, grid))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("data", ["random", "positive", "constant"])
+def test_g_and_gh_keep_fp32(pg, cuda, data):
+    """G and G^H alone against the FP64 operator: taps of 1 on 3 x 5 cells, so
+    that nothing but the values' own splits, products and sums is off.  A
+    rounding of FP32 is 2.5e-8 in the mean square; a cell passes one product, one
+    block sum and two or three sums outside, 5e-8 or less in all.  Tolerance
+    1e-7 (relative L2): values cut to 23 bits without their low x low products
+    are 1.3e-7 off on random and 2.0e-7 on constant values."""
+    torch = cuda
+    n, M = 64, 20000
+    rng = np.random.default_rng(3)
+    u, v = rng.uniform(-n, n, M), rng.uniform(-n, n, M)
+
+    def values(size):
+        if data == "random":
+            z = rng.standard_normal(size) + 1j * rng.standard_normal(size)
+        elif data == "positive":
+            z = rng.random(size) + 1j * rng.random(size)
+        else:
+            z = np.full(size, 1.2345678 + 0.7654321j)
+        return torch.from_numpy(z).to(torch.complex64).cuda()
+    g, y = values(4 * n * n), values(M)
+    out = {}
+    for prec, dt in (("fp32", torch.complex64), ("fp64", torch.complex128)):
+        op = pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, kernel="box",
+                                    Ju=3, Jv=5, precision=prec)
+        vis = torch.empty(M, dtype=dt, device="cuda")
+        grid = torch.empty(4 * n * n, dtype=dt, device="cuda")
+        op.degrid_into(g.to(dt), vis)
+        op.grid_into(y.to(dt), grid)
+        out[prec] = vis.cpu().numpy(), grid.cpu().numpy()
+    for a, b in zip(out["fp32"], out["fp64"]):
+        assert rel_l2(a, b) < 1e-7
