@@ -24,7 +24,7 @@
 // 1.66e-7.
 //
 // What bounds them: on paper the mma rate, measured 0.5 a cycle and SM.  A 1024^2
-// image with 10^6 rows of 4 to 24 taps takes 210 us (G) and 280 (G^H), 269 and 542
+// image with 10^6 rows of 4 to 24 taps takes 215 us (G) and 280 (G^H), 269 and 542
 // with the band kernels, 187 and 261 with two TF32 pieces of 11 bits, which lost
 // precision (1.0e-7 in G).  The registers of the blocks and shared memory leave
 // 10 to 14 warps an SM, whose chains of dependent products and splits are the
@@ -516,10 +516,10 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
 // The factors (term g, columns 8 j + t and 8 j + t + 4) are the 16 x 8
 // operand, the grid's real and then its imaginary parts the 8 x 8 one.  The
 // TV blocks are independent chains, unrolled together.
-template <int TV, int TM>
+template <bool SCALED, int TV, int TM>
 __device__ __forceinline__ void degrid_oct_rows(float2 (&T)[TM][2], const float4 (*B)[32],
                                                 const float2 (*ring)[8 * (TM + 1) * 8], int base,
-                                                int row0, int tu, int g, int t) {
+                                                int row0, int tu, int g, int t, float up) {
   // not unrolled: with every shape's columns unrolled the code outgrows the
   // instruction cache
 #pragma unroll 1
@@ -532,9 +532,22 @@ __device__ __forceinline__ void degrid_oct_rows(float2 (&T)[TM][2], const float4
     const Split f = split<true>(make_float2(v.x, v.y), make_float2(v.z, v.w));
     // (bx + i by) (gr + i gi): the rows (bx, by) times gr, (-by, bx) times gi
     const Rows a = rows(f.re, f.im, negate(f.im), f.re);
+    float2 g0[TV], g1[TV];
+#pragma unroll
+    for (int i = 0; i < TV; ++i) {
+      g0[i] = blk[64 * i];
+      g1[i] = blk[64 * i + other];
+    }
+    if constexpr (SCALED) {
+#pragma unroll
+      for (int i = 0; i < TV; ++i) {
+        g0[i] = make_float2(g0[i].x * up, g0[i].y * up);
+        g1[i] = make_float2(g1[i].x * up, g1[i].y * up);
+      }
+    }
     Split grid[TV];
 #pragma unroll
-    for (int i = 0; i < TV; ++i) grid[i] = split<false>(blk[64 * i], blk[64 * i + other]);
+    for (int i = 0; i < TV; ++i) grid[i] = split<false>(g0[i], g1[i]);
     float c[TV][4];
     multiply<TV>(c, [&](int) -> const Rows & { return a; },
                  [&](int i) -> const Split & { return grid[i]; });
@@ -642,6 +655,9 @@ __global__ void __launch_bounds__(kDegridWarps * 32, 14 / kDegridWarps) wstrip_d
   int place = 0;  // stage of the current oct
   int o = goct[0] + warp, oe = goct[1];
   int before = 1;  // octs that this warp took from the last group
+  float up = 1.f;   // scale of the grid's values
+  int looked = -1;  // the group in which `top`, the largest of them, was looked up
+  unsigned top = 0;
   for (int grp = 0; grp < tk.groups; ++grp) {
     const int oe1 = grp + 1 < tk.groups ? goct[grp + 2] : 0;
     // the block column that this group adds was committed a group ago, before
@@ -664,54 +680,82 @@ __global__ void __launch_bounds__(kDegridWarps * 32, 14 / kDegridWarps) wstrip_d
       const float4(*B)[32] = reinterpret_cast<const float4(*)[32]>(&st.B[0][lane]);
       const int4 term = st.term[lane];
       const int tv = term.w & 15, tu = (term.w >> 4) & 15, row0 = (term.w >> 8) & 1 ? 8 : 0;
-      float2 T[TM][2];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) T[i][0] = T[i][1] = make_float2(0.f, 0.f);
       const float2(*rg)[ROWS * 8] = ring;
-      bool todo = true;
-      if constexpr (TM >= 4)
-        if (tv == 4) degrid_oct_rows<4, TM>(T, B, rg, base, row0, tu, g, t), todo = false;
-      if constexpr (TM >= 3)
-        if (tv == 3) degrid_oct_rows<3, TM>(T, B, rg, base, row0, tu, g, t), todo = false;
-      if constexpr (TM >= 2)
-        if (tv == 2) degrid_oct_rows<2, TM>(T, B, rg, base, row0, tu, g, t), todo = false;
-      if (todo) degrid_oct_rows<1, TM>(T, B, rg, base, row0, tu, g, t);
-      float2 y = make_float2(0.f, 0.f);
+      float2 y;
+      bool cells = false;  // each term again over its own cells
+#pragma unroll 1
+      for (;;) {
+        float2 T[TM][2];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        if (i >= tv) break;  // the rest of the stage is an older oct's
-        const float4 A = st.A[i][lane];
-        y.x = fmaf(A.x, T[i][0].x, fmaf(-A.y, T[i][1].x, y.x));
-        y.y = fmaf(A.x, T[i][1].x, fmaf(A.y, T[i][0].x, y.y));
-        y.x = fmaf(A.z, T[i][0].y, fmaf(-A.w, T[i][1].y, y.x));
-        y.y = fmaf(A.z, T[i][1].y, fmaf(A.w, T[i][0].y, y.y));
+        for (int i = 0; i < TM; ++i) T[i][0] = T[i][1] = make_float2(0.f, 0.f);
+        auto product = [&](auto scaled) {
+          constexpr bool SCALED = decltype(scaled)::value;
+          if constexpr (TM >= 4)
+            if (tv == 4) return degrid_oct_rows<SCALED, 4, TM>(T, B, rg, base, row0, tu, g, t, up);
+          if constexpr (TM >= 3)
+            if (tv == 3) return degrid_oct_rows<SCALED, 3, TM>(T, B, rg, base, row0, tu, g, t, up);
+          if constexpr (TM >= 2)
+            if (tv == 2) return degrid_oct_rows<SCALED, 2, TM>(T, B, rg, base, row0, tu, g, t, up);
+          degrid_oct_rows<SCALED, 1, TM>(T, B, rg, base, row0, tu, g, t, up);
+        };
+        if (up == 1.f)
+          product(std::false_type());
+        else
+          product(std::true_type());
+        y = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+          if (i >= tv) break;  // the rest of the stage is an older oct's
+          const float4 A = st.A[i][lane];
+          y.x = fmaf(A.x, T[i][0].x, fmaf(-A.y, T[i][1].x, y.x));
+          y.y = fmaf(A.x, T[i][1].x, fmaf(A.y, T[i][0].x, y.y));
+          y.x = fmaf(A.z, T[i][0].y, fmaf(-A.w, T[i][1].y, y.x));
+          y.y = fmaf(A.z, T[i][1].y, fmaf(A.w, T[i][0].y, y.y));
+        }
+#pragma unroll
+        for (int s = 1; s <= 2; s <<= 1) {
+          y.x += __shfl_xor_sync(0xffffffffu, y.x, s);
+          y.y += __shfl_xor_sync(0xffffffffu, y.y, s);
+        }
+        // Sums of 2^-80 up to 2^120, or 0 beside such sums, had all the bits of
+        // their operands' pieces.  Others: see whether the grid's values are
+        // scaled as they should be (by a power of two that brings the largest
+        // of them to 1, kept for the octs that follow).  10^6 rows on a
+        // 1024^2 image, values of 10^-30: 245 us, 215 of order 1; with each such
+        // oct's terms summed cell by cell 1,092.
+        const unsigned size = max(__float_as_uint(fabsf(y.x)), __float_as_uint(fabsf(y.y)));
+        const bool off = size - 0x17800000u >= 0x7b800000u - 0x17800000u && size != 0;
+        const bool any_off = __any_sync(0xffffffffu, off);
+        if (!any_off && __any_sync(0xffffffffu, size != 0)) break;
+        if (looked != grp) {
+          looked = grp;
+          top = 0;
+          for (int j = 0; j < TM; ++j) {
+            int place = base + j;
+            if (place >= RING) place -= RING;
+            for (int k = lane; k < ROWS * 8; k += 32) {
+              const float2 v = ring[place][k];
+              top = max(top, max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.y))));
+            }
+          }
+          top = __reduce_max_sync(0xffffffffu, top);
+        }
+        if (top == 0) break;
+        const float fit = __uint_as_float((254u - min(max(top >> 23, 1u), 253u)) << 23);
+        if (top < 0x7f800000u && fit != up) {
+          up = fit;
+          continue;
+        }
+        // an infinite or NaN grid value, which zero factors have spread over
+        // the oct, or a term whose own cells are far below the largest
+        cells = any_off;
+        break;
       }
       issue(st);
-#pragma unroll
-      for (int s = 1; s <= 2; s <<= 1) {
-        y.x += __shfl_xor_sync(0xffffffffu, y.x, s);
-        y.y += __shfl_xor_sync(0xffffffffu, y.y, s);
-      }
-      const unsigned size = max(__float_as_uint(fabsf(y.x)), __float_as_uint(fabsf(y.y)));
-      bool again = __any_sync(0xffffffffu, size >= 0x7b800000u);  // 2^120
-      if (!again && __all_sync(0xffffffffu, size < 0x17800000u)) {  // 2^-80
-        // nothing but small sums: are the grid values small too, not only 0?
-        unsigned top = 0;
-        for (int j = 0; j < TM; ++j) {
-          int place = base + j;
-          if (place >= RING) place -= RING;
-          for (int k = lane; k < ROWS * 8; k += 32) {
-            const float2 v = ring[place][k];
-            top = max(top, max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.y))));
-          }
-        }
-        top = __reduce_max_sync(0xffffffffu, top);
-        again = top > 0 && top < 0x12800000u;  // 2^-90
-      }
-      if (again) {
-        // An infinite, NaN or huge grid value, which zero factors have spread
-        // over the oct, or values too small for the split.  Each term again,
-        // over its own taps only.
+      // 1 / up
+      const float down = __uint_as_float((254u << 23) - __float_as_uint(up));
+      y = make_float2(y.x * down, y.y * down);
+      if (cells) {
         for (int u = 0; u < kOctTerms; ++u) {
           const Term x = load_term(a, int64_t(o) * kOctTerms + u);
           float2 sum = make_float2(0.f, 0.f);

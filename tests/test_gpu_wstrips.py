@@ -201,3 +201,66 @@ def test_g_and_gh_keep_fp32(pg, cuda, data):
         out[prec] = vis.cpu().numpy(), grid.cpu().numpy()
     for a, b in zip(out["fp32"], out["fp64"]):
         assert rel_l2(a, b) < 1e-7
+
+
+def _scaled_case(pg, w_rows):
+    n, M = 48, 4000
+    rng = np.random.default_rng(5)
+    u, v = rng.uniform(-n, n, M), rng.uniform(-n, n, M)
+    kw = (dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=9) if w_rows else
+          dict(kernel="kb", Ju=12, Jv=12))
+    w = _w(rng, M, 2 * n) if w_rows else None
+    ops = [pg.MeasurementOperator(u, v, w, None, n, n, 2.0, power_iters=0, precision=p, **kw)
+           for p in ("fp32", "fp64")]
+    return ops, rng, n, M, u, v
+
+
+def _apply(torch, op, g, y, n, M):
+    vis = torch.empty(M, dtype=op.complex_dtype, device="cuda")
+    grid = torch.empty(4 * n * n, dtype=op.complex_dtype, device="cuda")
+    op.degrid_into(g.to(op.complex_dtype), vis)
+    op.grid_into(y.to(op.complex_dtype), grid)
+    return vis, grid
+
+
+@pytest.mark.parametrize("w_rows", [True, False])
+def test_values_of_any_scale(pg, cuda, w_rows):
+    """Powers of two scale G and G^H bit for bit: values far from 1 are brought
+    to it by powers of two, and the rest of the arithmetic has no scale.  (The
+    values span about 2^12, and the smallest results stay normal numbers.)"""
+    torch = cuda
+    (op, _), rng, n, M, _, _ = _scaled_case(pg, w_rows)
+    draw = lambda size: torch.from_numpy(np.exp(2j * np.pi * rng.random(size)) *  # noqa: E731
+                                         2.0 ** rng.uniform(-6, 6, size)).to(torch.complex64).cuda()
+    g, y = draw(4 * n * n), draw(M)
+    one = _apply(torch, op, g, y, n, M)
+    for e in (-84, -70, -40, 70, 95, 110):
+        got = _apply(torch, op, g * 2.0 ** e, y * 2.0 ** e, n, M)
+        for a, b in zip(got, one):
+            assert torch.equal(torch.view_as_real(a), torch.view_as_real(b) * 2.0 ** e), e
+
+
+@pytest.mark.parametrize("w_rows", [True, False])
+def test_scales_side_by_side(pg, cuda, w_rows):
+    """G where one half of the grid is 2^-100 of the other: visibilities whose
+    taps lie in the small half keep their own relative accuracy; and G^H of a
+    few visibilities of 2^70 among ones.  Zero grids give zeros.  Tolerance of
+    the file."""
+    torch = cuda
+    (op, ref), rng, n, M, u, v = _scaled_case(pg, w_rows)
+    N, S = 2 * n, 12
+    z = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    z[:, N // 2:] *= 2.0 ** -100
+    y = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    y[::97] *= 2.0 ** 70
+    g = torch.from_numpy(z.ravel()).to(torch.complex64).cuda()
+    y = torch.from_numpy(y).to(torch.complex64).cuda()
+    got, want = (_apply(torch, o, g, y, n, M) for o in (op, ref))
+    q = np.mod(np.floor(u - S / 2) + 1, N)
+    small = (q >= N // 2) & (q + S <= N)
+    assert small.sum() > 100
+    a, b = (t[0].cpu().numpy().astype(np.complex128) for t in (got, want))
+    assert rel_l2(a[small] * 2.0 ** 100, b[small] * 2.0 ** 100) < TOL
+    assert rel_l2(a[~small], b[~small]) < TOL
+    assert rel_l2(got[1].cpu().numpy(), want[1].cpu().numpy()) < TOL
+    assert _apply(torch, op, torch.zeros_like(g), y, n, M)[0].abs().max().item() == 0
