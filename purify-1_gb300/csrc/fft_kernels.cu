@@ -581,8 +581,10 @@ cudaError_t launch_fft_rows_inverse(const FftArgs &a, const void *grid, void *x,
 bool fft_cols_supported(int Nv, int W) {
   // at 4096 rows the block's registers would spill
   if (!fft_rows_supported(Nv) || Nv > 2048 || W <= 0) return false;
-  return W % (Nv >= 256 ? 8 : 16) == 0;
+  return W % col_block(Nv) == 0;
 }
+
+int fft_cols_blocks(int Nv, int W) { return W / col_block(Nv); }
 
 cudaError_t launch_fft_cols(bool inverse, const FftColArgs &c, cudaStream_t s) {
   if (!fft_cols_supported(c.Nv, c.W) || c.ld < c.W || (c.members && c.Nu <= 0) ||

@@ -60,6 +60,8 @@ struct FftColArgs {
 // True when the column pass handles W columns of height Nv.
 bool fft_cols_supported(int Nv, int W);
 cudaError_t launch_fft_cols(bool inverse, const FftColArgs &c, cudaStream_t s);
+// CTAs of the pass.
+int fft_cols_blocks(int Nv, int W);
 
 // The same passes over the channels of a batch that share one grid width Nu,
 // in one launch (blockIdx.y = member): channel members[k] of the ChannelIO<float>

@@ -859,6 +859,13 @@ void OperatorT<real>::degrid_slots(const void *grid, void *caller_vis) {
     WStripArgs a = strip_args_;
     a.grid = grid;
     a.vis_out = caller_vis ? caller_vis : ws_->slots;
+    // Not before the column pass is done where that leaves SMs empty: the tasks
+    // come in order of decreasing work, and the first of them, the longest,
+    // would all go there.  256^2 images (64 CTAs), rows of 4 to 24 taps, Phi in us
+    // with an early start and without: 10^5 rows 58.6, 45.5, 3 x 10^5 140.6, 108.9;
+    // 512^2 images (128 CTAs): 3 x 10^5 rows 96.6, 99.6; 128^2 (32): 8,000 rows 27.0, 29.0.
+    const int ahead = own_cols_ ? fft_cols_blocks(Nv_, Nu_) : 0;
+    a.early = ahead < 48 || ahead >= 120;
     mark_begin(kDegrid);
     cuda_check(launch_wstrip_degrid(a, ws_->stream), "w degrid");
     mark_end(kDegrid);

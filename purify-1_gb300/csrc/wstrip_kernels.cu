@@ -862,7 +862,7 @@ cudaError_t launch_strip(bool degrid, const WStripArgs &a, cudaStream_t s) {
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
   }
-  return launch_chain(fn, blocks, threads, smem, s, a);
+  return launch_chain_if(a.early, fn, blocks, threads, smem, s, a);
 }
 cudaError_t launch_tiles(bool degrid, const WStripArgs &a, cudaStream_t s) {
   if (a.ntasks == 0) return cudaSuccess;

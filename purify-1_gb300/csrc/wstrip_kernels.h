@@ -22,6 +22,7 @@ struct WStripArgs {
   int ntasks = 0, Nu = 0, Nv = 0;
   int tiles = 0, rows = 0;      // plan's tiles and rows
   bool wide = false;            // set by the launcher: the grid is read 16 bytes at a time
+  bool early = true;            // may start before the kernel ahead of it is done
 };
 
 struct WStripFoldArgs {
