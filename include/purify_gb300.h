@@ -126,6 +126,10 @@ typedef struct {
                             single-cell items, J <= 6), 2 = degrid then grid through the
                             slot-ordered buffer, 0 = default (one pass for J < 6); the
                             results are bit-identical */
+  int32_t row_kernels;   /* G and G^H of row-factor operators (w rows, supports of 9 to 32,
+                            Ju != Jv) in FP32: 1 = the band kernels, 2 = the tensor-core
+                            kernels, 3 = G with the former and G^H with the latter (2 and 3
+                            where supports and scratch allow), 0 = by estimated time */
 } purify_gb300_tuning;
 int purify_gb300_operator_create_tuned(const purify_gb300_create_args *args,
                                        const purify_gb300_tuning *tuning,
@@ -241,6 +245,8 @@ typedef struct {
   int64_t cell_group;      /* work-item shape: 1 one cell, 2 a 2 x 2 group, 3 a pair of a row */
   int64_t walk_tasks;      /* tasks of the column-walk G^H of Phi^H (0: it uses work items) */
   int64_t walk_steps;      /* column steps of the walk: sum over its columns of the fullest row */
+  int64_t row_kernels;     /* kernels of a row-factor operator, as in the tuning (1, 2 or 3; 0:
+                              it is none) */
 } purify_gb300_info;
 int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_info *info);
 

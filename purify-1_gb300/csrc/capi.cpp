@@ -130,6 +130,7 @@ pg::OperatorConfig to_config(const purify_gb300_create_args *a, const purify_gb3
     c.fft_columns = t->fft_columns;
     c.grid_walk = t->grid_walk;
     c.normal_pass = t->normal_pass;
+    c.row_kernels = t->row_kernels;
   }
   if (a->precision != PURIFY_GB300_FP32 && a->precision != PURIFY_GB300_FP64)
     throw pg::Error(pg::kInvalidArgument, "unknown precision");
@@ -395,6 +396,7 @@ int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_inf
     info->cell_group = i.cell_group;
     info->walk_tasks = i.walk_tasks;
     info->walk_steps = i.walk_steps;
+    info->row_kernels = i.row_kernels;
   });
 }
 

@@ -172,15 +172,18 @@ class OperatorT final : public Operator {
   int fold_J_ = 0, fold_Jv_ = 0;
   DeviceBuffer wcode_, wfactor_, wfactors_, wchunks_, wtask_chunk_;
   int wchunk_values_ = 0;
-  // Row factors on the tensor-core kernels (FP32): the strip plan's state.
-  // Visibilities are read and written in caller order; ws->slots, where it
-  // is used (the normal operator), then holds them in caller order too.
-  bool strips_ = false;
+  // Row factors on the tensor-core kernels (FP32), G^H or both directions: the
+  // strip plan's state.  Visibilities are then read and written in caller order,
+  // by the band kernels' G too; ws->slots, where it is used (the normal
+  // operator), holds them in caller order.
+  bool strip_g_ = false, strip_gh_ = false;
   int64_t strip_cells_ = 0;  // cells of all task windows
   WStripArgs strip_args_;
   WStripFoldArgs strip_fold_;
   DeviceBuffer stasks_, sorder_, sgroup_oct_, sterms_, sowner_;
   void init_strips(const WStripPlan &plan, int64_t &bytes);
+  // the row factors: wfactors_ after kStripSlack values where strips are in use
+  C *wfactors() const { return wfactors_.as<C>() + (strip_gh_ ? kStripSlack : 0); }
   int64_t nnz_ = 0, occupied_ = 0, work_items_ = 0, factor_values_ = 0;
   void init_plain(const OperatorConfig &cfg, int64_t &bytes, AxisTiling &tu, AxisTiling &tv,
                   std::vector<int32_t> &tile_tasks);
@@ -342,7 +345,7 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   // split weights are applied to the slot-ordered buffer before G^H, and the
   // column walk reads its own slot order
   if (split_weights_ || walk_) fused_adjoint_ = false;
-  if (strips_) fused_forward_ = fused_adjoint_ = true;
+  if (strip_gh_) fused_forward_ = fused_adjoint_ = true;
   ntu_ = tu.n;
   ntv_ = tv.n;
   slot_stride_ = int64_t(win_rows_) * win_cols_;
@@ -394,13 +397,13 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   cufft_check(cufftPlan2d(&fft_, Nv_, Nu_, Traits<real>::kType), "cufftPlan2d");
   fft_ok_ = true;
   if (sizeof(real) == 4 && fft_rows_supported(Nu_)) {
-    const std::vector<float> twu = strips_ ? fft_twiddle_table(Nu_) : fft_twiddles(Nu_);
+    const std::vector<float> twu = strip_gh_ ? fft_twiddle_table(Nu_) : fft_twiddles(Nu_);
     tw_u_.alloc(sizeof(float) * twu.size(), &bytes);
     tw_u_.upload(twu.data(), sizeof(float) * twu.size(), stream_);
     own_cols_ = cfg.fft_columns != 1 && fft_cols_supported(Nv_, Nu_);
     std::vector<float> twv;
     if (own_cols_) {
-      twv = strips_ ? fft_twiddle_table(Nv_) : fft_twiddles(Nv_);
+      twv = strip_gh_ ? fft_twiddle_table(Nv_) : fft_twiddles(Nv_);
       tw_v_.alloc(sizeof(float) * twv.size(), &bytes);
       tw_v_.upload(twv.data(), sizeof(float) * twv.size(), stream_);
     } else {
@@ -448,18 +451,19 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   info_.fp64 = cfg.fp64;
   info_.kernel = cfg.kernel;
   info_.w_term = cfg.w_term;
-  info_.tasks = strips_ ? strip_args_.ntasks : ntasks_;
+  info_.tasks = strip_gh_ ? strip_args_.ntasks : ntasks_;
   info_.device_bytes = bytes;
   info_.kernel_fit_error = wmode_ ? 0.0 : fit.max_error;
   info_.nnz = nnz_;
   info_.occupied_cells = occupied_;
   info_.work_items = work_items_;
   info_.slots = S_;
-  info_.window_cells = strips_ ? strip_cells_ / strip_args_.ntasks : slot_stride_;
+  info_.window_cells = strip_gh_ ? strip_cells_ / strip_args_.ntasks : slot_stride_;
   info_.factor_values = factor_values_;
   info_.cell_group = group_;
   info_.walk_tasks = walk_ ? walk_ntasks_ : 0;
   info_.walk_steps = walk_ ? walk_steps_ : 0;
+  info_.row_kernels = !wmode_ ? 0 : strip_g_ ? 2 : strip_gh_ ? 3 : 1;
 
   set_norm(1.0);
   if (cfg.power_iters > 0) power_method(cfg.power_iters, cfg.power_tol);
@@ -700,15 +704,16 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
   tv = plan.tv;
   tile_tasks = plan.tile_tasks;
   if constexpr (sizeof(real) == 4) {
-    // The tensor-core kernels wherever their windows fit in the scratch of
-    // the band kernels' (the sizes callers see stay those), which is always so
-    // but for grids of a few groups.  Measured on a 1024^2 image with 2 x 10^6
-    // rows of 4 to 24 taps: Phi 541 us with the band kernels, 336 with these;
-    // Phi^H 1043, 395.  With 5 x 10^4 rows: 80, 83; 144, 109.
+    // The tensor-core kernels by direction, by their estimated times, where their
+    // windows fit in the scratch of the band kernels' (the sizes callers see stay
+    // those): G^H alone, or both.
     WStripPlan strips;
-    if (M_ > 0 && build_wstrips(plan, int64_t(win_rows_) * win_cols_ * ntasks_, strips)) {
-      init_strips(strips, bytes);
-      strips_ = true;
+    if (M_ > 0 && cfg.row_kernels != 1 &&
+        build_wstrips(plan, int64_t(win_rows_) * win_cols_ * ntasks_, strips)) {
+      const RowKernels k = choose_row_kernels(plan, strips);
+      strip_gh_ = cfg.row_kernels == 0 ? k.gh : true;
+      strip_g_ = strip_gh_ && (cfg.row_kernels == 0 ? k.g : cfg.row_kernels == 2);
+      if (strip_gh_) init_strips(strips, bytes);
     }
   }
   S_ = M_;
@@ -719,7 +724,7 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
   work_items_ = M_;
   // state of the band kernels (the strip plan's terms carry theirs)
   std::vector<C> wt;
-  if (!strips_) {
+  if (!strip_g_) {
     wt.resize(M_);
     for (int64_t i = 0; i < M_; ++i)
       wt[i] = C(real(plan.weight[i].real()), real(plan.weight[i].imag()));
@@ -750,9 +755,9 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
   // The strip kernels form addresses up to 48 values past a row's factors and
   // 16 before them (for copies of nothing): the strip plan's offsets start at
   // kStripSlack, and as many values follow the last.
-  const int64_t slack = strips_ ? kStripSlack : 0;
+  const int64_t slack = strip_gh_ ? kStripSlack : 0;
   wfactors_.alloc(sizeof(C) * (plan.factor_count + 2 * slack + 2), &bytes);
-  strip_args_.factors = wfactors_.as<C>() + slack;
+  strip_args_.factors = wfactors();
   cuda_check(cudaMemset(wfactors_.get(), 0, sizeof(C) * (plan.factor_count + 2 * slack + 2)),
              "memset");
   const int64_t chunk_rows = 1 << 20;
@@ -763,7 +768,7 @@ void OperatorT<real>::init_w(const OperatorConfig &cfg, int64_t &bytes, AxisTili
     const int64_t f1 = i1 < M_ ? plan.factor[i1] : plan.factor_count;
     buf.resize(size_t(f1 - f0));
     wplan_factors<real>(plan, i0, i1, buf.data());
-    cuda_check(cudaMemcpy(wfactors_.as<C>() + slack + f0, buf.data(), sizeof(C) * (f1 - f0),
+    cuda_check(cudaMemcpy(wfactors() + f0, buf.data(), sizeof(C) * (f1 - f0),
                           cudaMemcpyHostToDevice),
                "factor upload");
   }
@@ -855,7 +860,7 @@ void OperatorT<real>::release(cudaStream_t user) {
 
 template <typename real>
 void OperatorT<real>::degrid_slots(const void *grid, void *caller_vis) {
-  if (strips_) {
+  if (strip_g_) {
     WStripArgs a = strip_args_;
     a.grid = grid;
     a.vis_out = caller_vis ? caller_vis : ws_->slots;
@@ -878,9 +883,10 @@ void OperatorT<real>::degrid_slots(const void *grid, void *caller_vis) {
     w.order = task_order_.as<int32_t>();
     w.code = wcode_.as<int32_t>();
     w.factor = wfactor_.as<int64_t>();
-    w.factors = wfactors_.get();
+    w.factors = wfactors();
     w.weight = weight_.get();
-    w.slot_out = ws_->slots;
+    w.slot_out = caller_vis ? caller_vis : ws_->slots;
+    w.slot_user = strip_gh_ ? slot_user_.as<int32_t>() : nullptr;
     w.chunks = wchunks_.as<WChunk>();
     w.task_chunk = wtask_chunk_.as<int32_t>();
     w.chunk_values = wchunk_values_;
@@ -932,7 +938,7 @@ void OperatorT<real>::grid_slots(void *grid, const void *caller_vis) {
 template <typename real>
 void OperatorT<real>::grid_core(void *grid, const void *vis, const int32_t *slot_user,
                                 void *windows) {
-  if (strips_) {
+  if (strip_gh_) {
     WStripArgs a = strip_args_;
     a.vis_in = vis;
     a.windows = windows;
@@ -954,7 +960,7 @@ void OperatorT<real>::grid_core(void *grid, const void *vis, const int32_t *slot
     w.order = task_order_.as<int32_t>();
     w.code = wcode_.as<int32_t>();
     w.factor = wfactor_.as<int64_t>();
-    w.factors = wfactors_.get();
+    w.factors = wfactors();
     w.weight = weight_.get();
     w.slot_in = vis;
     w.chunks = wchunks_.as<WChunk>();
@@ -1079,7 +1085,7 @@ FftArgs OperatorT<real>::fft_args() const {
   f.su = reinterpret_cast<const float *>(su_active());
   f.sv = reinterpret_cast<const float *>(sv_d_.get());
   f.tw_u = tw_u_.get();
-  f.tw_table = strips_;
+  f.tw_table = strip_gh_;
   return f;
 }
 
@@ -1110,7 +1116,7 @@ FftColArgs OperatorT<real>::col_args(const void *in, void *out) const {
   c.y0 = y0_;
   c.Ny = Ny_;
   c.tw_v = tw_v_.get();
-  c.tw_table = strips_;
+  c.tw_table = strip_gh_;
   return c;
 }
 
@@ -1703,6 +1709,8 @@ std::unique_ptr<Operator> Operator::create(const OperatorConfig &cfg) {
   if (cfg.cell_group >= 2 && (cfg.fp64 || cfg.Ju > kMaxGroupJ || cfg.w_term || cfg.Ju != cfg.Jv))
     throw Error(kUnsupported,
                 "2 x 2 and row-pair work items need complex<float>, J <= 6 and no w-projection");
+  if (cfg.row_kernels < 0 || cfg.row_kernels > 3)
+    throw Error(kInvalidArgument, "row_kernels must be 0 (automatic), 1, 2 or 3");
   if (cfg.w_term && (cfg.M > 0 && !cfg.w))
     throw Error(kInvalidArgument, "w-projection needs the w coordinates");
   if (cfg.w_term && (cfg.Jw < 1 || cfg.Jw + cfg.Ju - 1 > kMaxWSupport) && !cfg.jw_rows)

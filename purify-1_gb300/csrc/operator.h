@@ -67,6 +67,7 @@ struct OperatorConfig {
   // no slot vector, but holds two J x J register blocks (194 registers at
   // J = 6, where it measured slower).
   int normal_pass = 0;
+  int row_kernels = 0;
 };
 
 // A plan fraction t + d (see PlanRequest::group) in precision `real`, kept
@@ -90,6 +91,7 @@ struct OperatorInfo {
   int device = 0;
   int64_t slots = 0, window_cells = 0, factor_values = 0, cell_group = 1;
   int64_t walk_tasks = 0, walk_steps = 0;
+  int64_t row_kernels = 0;
 };
 
 // Scratch of one apply held outside the operator, so that several applies of

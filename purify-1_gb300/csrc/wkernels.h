@@ -22,7 +22,8 @@ struct WArgs {
   const int64_t *factor = nullptr; // per visibility: first factor (complex index)
   const void *factors = nullptr;   // complex factors A_0..A_2, B_0..B_2 per row
   const void *weight = nullptr;    // per visibility, complex, phase sign folded in
-  void *slot_out = nullptr;        // degrid output in plan order
+  void *slot_out = nullptr;        // degrid output in plan order, or through slot_user
+  const int32_t *slot_user = nullptr;  // degrid, FP32: output index of each visibility
   const void *slot_in = nullptr;   // grid input in plan order
   const WChunk *chunks = nullptr;  // staging chunks (wplan.h)
   const int32_t *task_chunk = nullptr;

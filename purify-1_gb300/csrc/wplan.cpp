@@ -233,7 +233,7 @@ WPlan build_wplan(const WPlanRequest &rq) {
   return P;
 }
 
-bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
+bool build_wstrips(const WPlan &plan, int64_t max_cells, WStripPlan &out) {
   WStripPlan W;
   const int64_t M = plan.M;
   W.tiles = (plan.Smax + 7 + 7) / 8;
@@ -277,13 +277,7 @@ bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
                      [&](int32_t x, int32_t y) { return key[x] < key[y]; });
 
   // Octs of every group: the terms of a row stay together, an oct stays in
-  // one half.  Rows are named by their position in the new order.
-  std::vector<int64_t> factor(M);
-  int64_t off = 0;
-  for (int64_t r = 0; r < M; ++r) {
-    factor[r] = off;
-    off += int64_t(2) * wrow_rank(plan.code[order[r]]) * wrow_support(plan.code[order[r]]);
-  }
+  // one half.
   std::vector<int32_t> goct(ngroups + 1, 0);  // first oct of each group
   std::vector<int64_t> cost(ngroups, 0);
   const WTerm none{0, 0, -1, 0.f, 0.f, 0, 0};
@@ -306,7 +300,7 @@ bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
       const int tu = std::max((*oct >> 4) & 15, 15 - (key[i] & 15));
       for (int e = 0; e < rank; ++e) {
         WTerm &t = W.terms[(W.octs.size() - 1) * kOctTerms + used + e];
-        t.a = factor[r] + int64_t(e) * S;
+        t.a = plan.factor[i] + int64_t(e) * S;
         t.b_off = rank * S;
         t.m = plan.slot_user[i];
         t.wx = float(plan.weight[i].real());
@@ -402,7 +396,8 @@ bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
   }
   W.order.resize(W.tasks.size());
   std::iota(W.order.begin(), W.order.end(), 0);
-  std::vector<int64_t> tcost(W.tasks.size(), 0);
+  std::vector<int64_t> &tcost = W.task_cost;
+  tcost.assign(W.tasks.size(), 0);
   for (size_t k = 0; k < W.tasks.size(); ++k) {
     const WStripTask &t = W.tasks[k];
     tcost[k] = 4 * t.groups;
@@ -412,27 +407,66 @@ bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out) {
   std::stable_sort(W.order.begin(), W.order.end(),
                    [&](int32_t x, int32_t y) { return tcost[x] > tcost[y]; });
 
-  // The plan's rows in strip order.
-  auto permute = [&](auto &v) {
-    auto old = v;
-#pragma omp parallel for schedule(static)
-    for (int64_t r = 0; r < M; ++r) v[r] = old[order[r]];
-  };
-  permute(plan.code);
-  permute(plan.weight);
-  permute(plan.slot_user);
-  permute(plan.gen_u);
-  permute(plan.gen_v);
-  permute(plan.gen_w);
-  permute(plan.gen_jw);
-  plan.factor = factor;
-  for (int64_t r = 0; r < M; ++r) plan.user_slot[plan.slot_user[r]] = int32_t(r);
-  plan.tasks.clear();
-  plan.task_order.clear();
-  plan.chunks.clear();
-  plan.task_chunk.assign(1, 0);
   out = std::move(W);
   return true;
+}
+
+// Each launch takes about fixed + max(A, B) + alpha min(A, B) us: A the work of
+// all tasks, B the longest task's.  The band kernels' work goes by the steps
+// their warps take over a row's taps, as many as 18 of them spent on a row
+// besides, and by window cells; the strip kernels' by octets, their blocks,
+// groups or window cells: they waste octets that few rows fill and columns that
+// no row touches.  Fitted separately below and at four blocks (whose code starts
+// slowly) to both kernels' times on 121 coverages: 64^2 to 1024^2 images, also
+// 624 x 208 and 150 x 900, 2 x 10^3 to 10^6 rows, uniform and peaked, supports of 4 to
+// 24; rms errors of the fits 4 to 12%.  The strip kernels are taken where
+// they are expected to win by 3%.  Some of the times, us, band and strip
+// kernels: 512^2, 3 x 10^4 rows of 4 to 24 taps: G 24, 30, G^H 48, 45; 10^6: 282, 180 and
+// 557, 246; 1024^2, 10^5: 61, 74 and 132, 126; 3 x 10^5: 111, 119 and 219, 152; 624 x 208,
+// 8,000: 16, 16 and 23, 33; supports of 9, 400^2, 2,000: 11, 13 and 17, 17; 2 x 10^5: 80,
+// 27 and 174, 39.
+RowKernels choose_row_kernels(const WPlan &P, const WStripPlan &W) {
+  double steps = 0, longest = 0;
+  for (const Task &t : P.tasks) {
+    double c = 0;
+    for (int32_t i = t.batch_begin; i < t.batch_end; ++i) {
+      // rows of taps that the 32 lanes take at once
+      const int S = wrow_support(P.code[i]), at_once = std::max(1, 32 / S);
+      c += 18 + wrow_rank(P.code[i]) * ((S + at_once - 1) / at_once);
+    }
+    steps += c;
+    longest = std::max(longest, c);
+  }
+  const double windows = double(P.win_rows) * P.win_cols * double(P.tasks.size());
+  double blocks = 0, groups = 0, slongest = 0;
+  for (int32_t o : W.octs) blocks += (o & 15) * ((o >> 4) & 15);
+  for (size_t k = 0; k < W.tasks.size(); ++k) {
+    groups += W.tasks[k].groups;
+    slongest = std::max(slongest, double(W.task_cost[k]));
+  }
+  const double octs = double(W.octs.size()), swindows = double(W.window_cells),
+               cells = double(P.Nu) * P.Nv;
+  auto time = [](double fixed, double a, double b, double alpha) {
+    return fixed + std::max(a, b) + alpha * std::min(a, b);
+  };
+  double band_g, band_gh, strip_g, strip_gh;
+  if (W.tiles >= 4) {
+    band_g = time(5.9, 8.0e-6 * steps + 1.75e-6 * windows, 3.15e-3 * longest, 0.39);
+    band_gh = time(12.3, 1.58e-5 * steps + 3.7e-6 * windows + 1.2e-6 * cells, 7.8e-3 * longest,
+                   0.24);
+    strip_g = time(8.3, 6.4e-4 * octs + 3.9e-5 * blocks + 6.7e-4 * groups, 0.068 * slongest, 0.36);
+    strip_gh = time(17.9, 7.5e-4 * octs + 6.4e-5 * blocks + 1.24e-6 * swindows + 4.2e-6 * cells,
+                    0.168 * slongest, 0.19);
+  } else {
+    band_g = time(4.9, 6.7e-6 * steps + 1.8e-6 * windows, 3.0e-3 * longest, 0.7);
+    band_gh = time(11.3, 1.44e-5 * steps + 4.2e-6 * windows + 1.5e-6 * cells, 4.1e-3 * longest, 1);
+    strip_g = time(6.1, 4.0e-4 * octs, 0.097 * slongest, 0.96);
+    strip_gh = time(0.8, 5.7e-4 * octs + 9.6e-7 * swindows + 1.4e-5 * cells, 0.112 * slongest, 1);
+  }
+  RowKernels r;
+  r.gh = strip_gh < 0.97 * band_gh;
+  r.g = r.gh && strip_g < 0.97 * band_g;
+  return r;
 }
 
 template <typename T>

@@ -104,16 +104,22 @@ struct WStripPlan {
   std::vector<int32_t> order;        // launch order: most work first
   std::vector<int32_t> group_oct;    // per task its groups + 1 offsets into octs
   std::vector<int32_t> octs;         // tv | tu << 4 | half << 8 | terms << 12
+  std::vector<int64_t> task_cost;    // blocks of a task's octs, and 4 for each group
   std::vector<WTerm> terms;          // 8 per oct
   std::vector<int2_t> owner;         // strips x cols: tasks [x, y) that hold the group
   int64_t window_cells = 0;          // complex cells of all task windows
 };
 
-// Reorders the rows of `plan` into strip order (its tasks and chunks, which
-// name rows by their old order, are emptied) and builds the strip plan, with
-// task windows of at most max_cells complex cells in all.  Returns false, with
-// `plan` untouched, where that is not possible.
-bool build_wstrips(WPlan &plan, int64_t max_cells, WStripPlan &out);
+// Builds the strip plan of `plan`'s rows, with task windows of at most max_cells
+// complex cells in all.  Returns false where that is not possible.
+bool build_wstrips(const WPlan &plan, int64_t max_cells, WStripPlan &out);
+
+// Which of the two directions the strip kernels are expected to take less time
+// for than the band kernels.
+struct RowKernels {
+  bool g = false, gh = false;
+};
+RowKernels choose_row_kernels(const WPlan &plan, const WStripPlan &strips);
 
 // Fields of a row code: the support S and the mask of stored terms (bit r:
 // term r of the sample matrix is nonzero); the rank is the mask's popcount.

@@ -56,7 +56,8 @@ class Tuning(ctypes.Structure):
                 ("tile", ctypes.c_int32), ("fused_permute", ctypes.c_int32),
                 ("cell_group", ctypes.c_int32), ("class_cap", ctypes.c_int32),
                 ("keep_store", ctypes.c_int32), ("fft_columns", ctypes.c_int32),
-                ("grid_walk", ctypes.c_int32), ("normal_pass", ctypes.c_int32)]
+                ("grid_walk", ctypes.c_int32), ("normal_pass", ctypes.c_int32),
+                ("row_kernels", ctypes.c_int32)]
 
 
 class Info(ctypes.Structure):
@@ -70,6 +71,7 @@ class Info(ctypes.Structure):
         ("norm", ctypes.c_double), ("slots", ctypes.c_int64), ("window_cells", ctypes.c_int64),
         ("factor_values", ctypes.c_int64), ("cell_group", ctypes.c_int64),
         ("walk_tasks", ctypes.c_int64), ("walk_steps", ctypes.c_int64),
+        ("row_kernels", ctypes.c_int64),
     ]
 
 
@@ -485,7 +487,8 @@ class MeasurementOperator:
                        int(tuning.get("tile", 0)), int(tuning.get("fused_permute", -1)),
                        int(tuning.get("cell_group", 0)), int(tuning.get("class_cap", 0)),
                        int(tuning.get("keep_store", 0)), int(tuning.get("fft_columns", 0)),
-                       int(tuning.get("grid_walk", 0)), int(tuning.get("normal_pass", 0)))
+                       int(tuning.get("grid_walk", 0)), int(tuning.get("normal_pass", 0)),
+                       int(tuning.get("row_kernels", 0)))
             _check(L.purify_gb300_operator_create_tuned(ctypes.byref(a), ctypes.byref(t),
                                                         ctypes.byref(h)))
         else:

@@ -150,7 +150,8 @@ def test_grids_and_visibilities_of_any_alignment(pg, cuda, w_rows):
     kw = (dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=9) if w_rows else
           dict(kernel="kb", Ju=12, Jv=12))
     op = pg.MeasurementOperator(u, v, _w(rng, M, N) if w_rows else None, None, n, n, 2.0,
-                                power_iters=0, precision="fp32", **kw)
+                                power_iters=0, precision="fp32", tuning={"row_kernels": 2}, **kw)
+    assert op.info()["row_kernels"] == 2
     z = torch.from_numpy(rng.standard_normal(2 * (N * N + M))).float().cuda()
     out = []
     for shift in (0, 1):
@@ -193,7 +194,8 @@ def test_g_and_gh_keep_fp32(pg, cuda, data):
     out = {}
     for prec, dt in (("fp32", torch.complex64), ("fp64", torch.complex128)):
         op = pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, kernel="box",
-                                    Ju=3, Jv=5, precision=prec)
+                                    Ju=3, Jv=5, precision=prec, tuning={"row_kernels": 2})
+        assert op.info()["row_kernels"] == (2 if prec == "fp32" else 1)
         vis = torch.empty(M, dtype=dt, device="cuda")
         grid = torch.empty(4 * n * n, dtype=dt, device="cuda")
         op.degrid_into(g.to(dt), vis)
@@ -210,8 +212,9 @@ def _scaled_case(pg, w_rows):
     kw = (dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=9) if w_rows else
           dict(kernel="kb", Ju=12, Jv=12))
     w = _w(rng, M, 2 * n) if w_rows else None
-    ops = [pg.MeasurementOperator(u, v, w, None, n, n, 2.0, power_iters=0, precision=p, **kw)
-           for p in ("fp32", "fp64")]
+    ops = [pg.MeasurementOperator(u, v, w, None, n, n, 2.0, power_iters=0, precision=p,
+                                  tuning={"row_kernels": 2}, **kw) for p in ("fp32", "fp64")]
+    assert ops[0].info()["row_kernels"] == 2
     return ops, rng, n, M, u, v
 
 
@@ -264,3 +267,52 @@ def test_scales_side_by_side(pg, cuda, w_rows):
     assert rel_l2(a[~small], b[~small]) < TOL
     assert rel_l2(got[1].cpu().numpy(), want[1].cpu().numpy()) < TOL
     assert _apply(torch, op, torch.zeros_like(g), y, n, M)[0].abs().max().item() == 0
+
+
+@pytest.mark.parametrize("row_kernels", [1, 2, 3])
+@pytest.mark.parametrize("Jw,M,ny,nx,dense,fits", [
+    (1, 1, 32, 32, False, True), (5, 900, 32, 45, False, True), (6, 2000, 32, 45, False, True),
+    (6, 2000, 33, 50, False, False), (13, 1500, 64, 40, True, True), (14, 1500, 64, 40, True, True),
+    (21, 1000, 48, 36, False, True), (22, 700, 48, 36, True, True), (29, 800, 31, 62, True, False)])
+def test_every_choice_of_kernels(pg, oracle_mod, cuda, row_kernels, Jw, M, ny, nx, dense, fits):
+    """The band kernels, the tensor-core kernels and G with the one, G^H with the
+    other, on both sides of each number of 8-cell blocks, also where the windows
+    would not fit and past the largest support (25), where all are the band
+    kernels; and the allocation-free entry point."""
+    torch = cuda
+    rng = np.random.default_rng(Jw)
+    u, v = rng.uniform(-nx, nx, M), rng.uniform(-ny, ny, M)
+    if dense:
+        u[: M // 2], v[: M // 2] = 3.25 + 0.5 * rng.random(M // 2), -5.75 + 0.5 * rng.random(M // 2)
+    wt = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    kw = dict(kernel="kb", Ju=4, Jv=4, w_term=True, Jw=Jw)
+    args = (u, v, _w(rng, M, 2 * nx), wt)
+    tuned = dict(kw, tuning={"row_kernels": row_kernels})
+    _check(pg, oracle_mod, cuda, args, tuned, kw, ny, nx, Jw)
+    op = pg.MeasurementOperator(*args, ny, nx, 2.0, power_iters=0, precision="fp32", **tuned)
+    assert op.info()["row_kernels"] == (row_kernels if fits else 1)
+    y = torch.from_numpy(rng.standard_normal(M) + 1j * rng.standard_normal(M)).to(
+        torch.complex64).cuda()
+    a, b = (torch.empty(4 * ny * nx, dtype=torch.complex64, device="cuda") for _ in range(2))
+    op.grid_into(y, a)
+    op.grid_no_alloc_into(y, b)
+    assert torch.equal(a, b)
+
+
+def test_kernels_chosen_by_coverage(pg, cuda):
+    """Few rows, or rows that are far apart, stay on the band kernels; rows that
+    fill the octets go to the tensor-core kernels, G^H before G.  (On either side
+    of the estimate the other choice costs about 20% or more.)"""
+    def chosen(n, M, core=0.7):
+        rng = np.random.default_rng(M)
+        c = rng.random(M) < core
+        u, v = (np.where(c, np.clip(rng.normal(0, 0.15 * 2 * n, M), -n, n - 1),
+                         rng.uniform(-n, n, M)) for _ in range(2))
+        w = rng.uniform(-1, 1, M) * 12 * 60.0 * 60.0 * 180.0 / (2 * n) / np.pi
+        jw = rng.integers(1, 22, M).astype(np.int32)
+        op = pg.MeasurementOperator(u, v, w, None, n, n, 2.0, power_iters=0, kernel="kb", Ju=4,
+                                    Jv=4, w_term=True, jw_rows=jw, precision="fp32")
+        return op.info()["row_kernels"]
+    assert chosen(256, 2000) == 1 and chosen(512, 2000) == 1
+    assert chosen(512, 300000) == 2 and chosen(128, 100000) == 2
+    assert chosen(1024, 100000, 1.0) == 3
