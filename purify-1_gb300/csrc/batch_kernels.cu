@@ -17,12 +17,12 @@ using namespace dev;
 // The element-wise grouped kernels run over a block map: block b works on
 // channel map[b].x, its block map[b].y, so no block is idle whatever the
 // spread of channel sizes.
-template <typename real>
-__global__ void __launch_bounds__(32 * FoldShape<real>::rows, sizeof(real) == 4 ? 8 : 4)
+template <typename real, int T, int R>
+__global__ void __launch_bounds__(32 * T, sizeof(real) == 4 ? 8 : 3)
     fold_group_kernel(const FoldArgs *__restrict__ folds, const int2 *__restrict__ map) {
   const int2 m = map[blockIdx.x];
   const FoldArgs &f = folds[m.x];
-  fold_tile<real>(f, fold_meta(f, m.y));
+  fold_tile<real, T, R>(f, fold_meta(f, m.y));
 }
 
 template <typename real>
@@ -182,7 +182,8 @@ cudaError_t launch_grid_group(const ApplyArgs<real> &a, const PolyTable<real> &p
 template <typename real>
 cudaError_t launch_fold_group(const FoldArgs *folds, const int2 *map, int nblocks, cudaStream_t s) {
   if (nblocks == 0) return cudaSuccess;
-  fold_group_kernel<real><<<nblocks, dim3(32, FoldShape<real>::rows), 0, s>>>(folds, map);
+  constexpr int T = sizeof(real) == 4 ? 4 : 8, R = sizeof(real) == 4 ? 8 : 4;
+  fold_group_kernel<real, T, R><<<nblocks, dim3(32, T), 0, s>>>(folds, map);
   return cudaGetLastError();
 }
 template <typename real>

@@ -83,13 +83,13 @@ __global__ void expand_kernel(const cplx<real> *__restrict__ in,
   }
 }
 
-template <typename real>
-__global__ void __launch_bounds__(32 * FoldShape<real>::rows, sizeof(real) == 4 ? 8 : 4)
+template <typename real, int T, int R, int MINB>
+__global__ void __launch_bounds__(32 * T, MINB)
     fold_kernel(const FoldArgs f) {
   dev::pdl_launch_next();
   const FoldTile m = fold_meta(f, int(blockIdx.x));  // the plan's, not a kernel's output
   dev::pdl_wait();  // the task windows are the previous kernel's output
-  fold_tile<real>(f, m);
+  fold_tile<real, T, R>(f, m);
 }
 
 template <typename real>
@@ -394,8 +394,14 @@ cudaError_t launch_walk_grid(const WalkArgs<real> &a, const PolyTable<real> &pol
 
 template <typename real>
 cudaError_t launch_fold(const FoldArgs &f, cudaStream_t s) {
-  return launch_chain(fold_kernel<real>, dim3(f.ntu * f.ntv), dim3(32, FoldShape<real>::rows), 0,
-                      s, f);
+  const dim3 tiles(f.ntu * f.ntv);
+  if constexpr (sizeof(real) == 4) {
+    if (f.ntu * f.ntv >= kFoldTiles)
+      return launch_chain(fold_kernel<real, 4, 8, 8>, tiles, dim3(32, 4), 0, s, f);
+    return launch_chain(fold_kernel<real, 8, 4, 4>, tiles, dim3(32, 8), 0, s, f);
+  } else {
+    return launch_chain(fold_kernel<real, 8, 4, 3>, tiles, dim3(32, 8), 0, s, f);
+  }
 }
 
 template <typename real>

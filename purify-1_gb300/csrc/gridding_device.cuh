@@ -1031,7 +1031,7 @@ __device__ __forceinline__ FoldTile fold_meta(const FoldArgs &f, int t) {
   return m;
 }
 
-// One CTA of 32 x FoldShape::rows threads per tile.  A cell sums, in this order, the
+// One CTA of 32 x T threads per tile.  A cell sums, in this order, the
 // windows of its own tile's tasks, then those of the tile above, the tile to
 // the left and the tile above-left, where their J - 1 halo rows / columns
 // reach into it.
@@ -1040,24 +1040,28 @@ __device__ __forceinline__ FoldTile fold_meta(const FoldArgs &f, int t) {
 // reads one window and some halos and is gone.  What helps is more bytes in
 // flight for each latency of that short life: the first window of each of the
 // four tiles is loaded before any is added (a 0 stands in for one that is not
-// there: a sum that began at +0 keeps its bits), and 128 threads hold 8 cells
-// each in FP32 (FP64: 256 threads of 2 cells, by registers).  Measured with cold caches against 256
+// there: a sum that began at +0 keeps its bits), and where there are many tiles
+// 128 threads hold 8 cells each.  Measured with cold caches against 256
 // threads of 4 cells that walked the four tiles one after the other: 31,520
 // tiles of 32^2 201 -> 100 us (4 TB/s), 17,408 of 32^2 101 -> 71, 7,880 of 48^2
 // 142 -> 94; one grid of 63 x 44 mostly ragged tiles 18.4 -> 14.8.
-template <typename real>
-struct FoldShape {
-  static constexpr int rows = sizeof(real) == 4 ? 4 : 8, cells = sizeof(real) == 4 ? 8 : 2;
-};
+// Fewer tiles than the chip has room for keep 256 threads of 4 cells, which are
+// done sooner: 484 tiles of 24^2 with halos of 23 9.3 us, 10.4 with 128 threads (one
+// walked after the other: 9.1), 121 tiles 8.2, 10.0 (8.2); 1,849 tiles 16.4, 14.2 (16.2);
+// tiles of 32^2, J = 4, 576: 8.0, 7.6 (8.1) but with the gridding before it 9.0, 11.5
+// (11.3); 1,024: 9.0, 8.3 (10.2).  FP64, by registers, 256 threads of 4 cells and 3
+// CTAs an SM at any size: 4,096 tiles 40.9, 4 CTAs of 2 cells each 55.5 (29 to 45 by the number
+// of tasks), 1,024 tiles 17.0, 19.2 (16.5), 361 tiles 10.9, 12.3 (13.2).
+constexpr int kFoldTiles = 800;  // FP32: from here 128 threads of 8 cells
 
 // A chunk of 32 columns from c0 and T * R rows from r0: thread (lq, ty) owns
 // rows ty + T r of column lq, in registers while the
 // task windows are walked.  For halos of at most 8 rows and 32 columns, which
 // then lie in r < 2 of the first chunks.  FULL: the whole chunk is in the tile.
-template <typename real, int R, bool FULL>
+template <typename real, int T, int R, bool FULL>
 __device__ __forceinline__ void fold_chunk(const FoldArgs &f, const FoldTile &m, int c0, int r0) {
   using C = cplx<real>;
-  constexpr int T = FoldShape<real>::rows, U = 8 / T;
+  constexpr int U = 8 / T;
   const int lq = c0 + int(threadIdx.x), lp = r0 + int(threadIdx.y);
   const int WWo = m.W + f.Ju - 1, WWl = m.Wl + f.Ju - 1;
   const int64_t ss = f.slot_stride;
@@ -1140,18 +1144,17 @@ __device__ __forceinline__ void fold_chunk(const FoldArgs &f, const FoldTile &m,
     if (col && row[r]) g[size_t(T * r) * ld] = s[r];
 }
 
-template <typename real>
+template <typename real, int T, int R>
 __device__ __forceinline__ void fold_tile(const FoldArgs &f, const FoldTile &m) {
   using C = cplx<real>;
-  constexpr int R = FoldShape<real>::cells, T = FoldShape<real>::rows;
   const int P = m.P, Q = m.Q, H = m.H, W = m.W, Hu = m.Hu, Wl = m.Wl;
   if (f.Jv <= 9 && f.Ju <= 33) {
     for (int c0 = 0; c0 < W; c0 += 32)
       for (int r0 = 0; r0 < H; r0 += T * R) {
         if (W - c0 >= 32 && H - r0 >= T * R)
-          fold_chunk<real, R, true>(f, m, c0, r0);
+          fold_chunk<real, T, R, true>(f, m, c0, r0);
         else
-          fold_chunk<real, R, false>(f, m, c0, r0);
+          fold_chunk<real, T, R, false>(f, m, c0, r0);
       }
     return;
   }

@@ -37,3 +37,40 @@ def test_fold_tiles(pg, oracle_mod, cuda, precision, tile, J, per_item, ny, nx, 
     want = ref.adjoint(y).reshape(ny, nx)
     assert torch.equal(out[0], out[1])
     assert rel_l2(out[0].cpu().numpy(), want) < (2e-6 if precision == "fp32" else 1e-12)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("n,tile,J,per_item", [
+    (112, 8, 4, 64), (120, 8, 4, 64), (117, 8, 8, 1), (112, 8, 8, 1)])
+def test_few_and_many_tiles(pg, oracle_mod, cuda, precision, n, tile, J, per_item):
+    """Single operators on both sides of the number of tiles from which CTAs have
+    128 threads (784 and 900, and ragged ones), halos up to a tile's width."""
+    torch = cuda
+    M = 4000
+    u, v = synthetic.mixed_uv(M, 2 * n, 2 * n, 0.5, 0.1, seed=n)
+    y = synthetic.random_vis(M, seed=J)
+    op = pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, kernel="kb", Ju=J,
+                                Jv=J, precision=precision,
+                                tuning={"tile": tile, "max_per_item": per_item})
+    ref = oracle_mod.Operator(u, v, None, None, n, n, 2.0, kernel="kb", Ju=J, Jv=J)
+    got = op.adjoint(torch.from_numpy(y).to(op.complex_dtype).cuda()).cpu().numpy()
+    assert rel_l2(got, ref.adjoint(y)) < (2e-6 if precision == "fp32" else 1e-12)
+
+
+@pytest.mark.parametrize("n", [64, 341])
+def test_wide_halos(pg, cuda, n):
+    """Halos of 23 cells (the walk over any halo) on few and on many tiles, against
+    the FP64 operator's G^H."""
+    torch = cuda
+    M = 3000
+    rng = np.random.default_rng(n)
+    u, v = rng.uniform(-n, n, M), rng.uniform(-n, n, M)
+    y = torch.from_numpy(synthetic.random_vis(M, seed=n)).to(torch.complex64).cuda()
+    out = []
+    for prec, dt in (("fp32", torch.complex64), ("fp64", torch.complex128)):
+        op = pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, kernel="kb",
+                                    Ju=20, Jv=20, precision=prec, tuning={"row_kernels": 1})
+        g = torch.empty(4 * n * n, dtype=dt, device="cuda")
+        op.grid_into(y.to(dt), g)
+        out.append(g.cpu().numpy())
+    assert rel_l2(out[0], out[1]) < 2e-6
