@@ -247,6 +247,9 @@ typedef struct {
   int64_t walk_steps;      /* column steps of the walk: sum over its columns of the fullest row */
   int64_t row_kernels;     /* kernels of a row-factor operator, as in the tuning (1, 2 or 3; 0:
                               it is none) */
+  int64_t degrid_warps;    /* warps per CTA of G, G^H and the one-pass normal operator (0: two */
+  int64_t grid_warps;      /* kernels); 0 for row-factor operators */
+  int64_t normal_warps;
 } purify_gb300_info;
 int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_info *info);
 

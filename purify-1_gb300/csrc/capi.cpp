@@ -397,6 +397,9 @@ int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_inf
     info->walk_tasks = i.walk_tasks;
     info->walk_steps = i.walk_steps;
     info->row_kernels = i.row_kernels;
+    info->degrid_warps = i.degrid_warps;
+    info->grid_warps = i.grid_warps;
+    info->normal_warps = i.normal_warps;
   });
 }
 

@@ -464,6 +464,11 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   info_.walk_tasks = walk_ ? walk_ntasks_ : 0;
   info_.walk_steps = walk_ ? walk_steps_ : 0;
   info_.row_kernels = !wmode_ ? 0 : strip_g_ ? 2 : strip_gh_ ? 3 : 1;
+  if (!wmode_) {
+    info_.degrid_warps = degrid_shape_.threads / 32;
+    info_.grid_warps = grid_shape_.threads / 32;
+    info_.normal_warps = one_pass_normal_ ? normal_shape_.threads / 32 : 0;
+  }
 
   set_norm(1.0);
   if (cfg.power_iters > 0) power_method(cfg.power_iters, cfg.power_tol);

@@ -92,6 +92,7 @@ struct OperatorInfo {
   int64_t slots = 0, window_cells = 0, factor_values = 0, cell_group = 1;
   int64_t walk_tasks = 0, walk_steps = 0;
   int64_t row_kernels = 0;
+  int64_t degrid_warps = 0, grid_warps = 0, normal_warps = 0;
 };
 
 // Scratch of one apply held outside the operator, so that several applies of

@@ -114,7 +114,12 @@ void balance_task_batches(Plan &P, int nw) {
 // coverages (64^2 to 1024^2 images, 4 x 10^3 to 10^7 visibilities, J = 2 to 8),
 // and a choice other than the default has to win by a margin.  Against the
 // defaults (`dealt`; 2 for the normal operator) G is 1.15, G^H 1.13 and the
-// normal operator 1.32 times as fast on average over these, and none slower.
+// normal operator 1.32 times as fast on average over these.
+// The warps that G^H's ordered flushes keep busy at once are fewer where a
+// flush is long and where registers leave few: with the 1500 of narrow supports
+// uniform and many-tiled coverages got more warps than were good for them
+// (336 coverages, us with the default, 4 warps: 724^2, 8 x 10^5, J = 8: 77, 101; J = 7: 61,
+// 75; 400^2, 2 x 10^5, uniform, J = 6: 21.5, 25.3), all of which keep the default now.
 // 512^2 image, 2 x 10^6 visibilities, J = 6: G 65 -> 35 us, G^H 131 -> 77;
 // J = 4: G 39 -> 29, G^H 67 -> 50, normal 90 -> 38.  G takes no fewer warps than
 // the default: on tiles of a batch or two they stage the window more slowly
@@ -156,7 +161,8 @@ PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) 
   };
   PlanWarps w;
   w.degrid = pick(dealt, dealt, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
-  w.grid = pick(dealt, dealt, 0.95, 1, 0, 1500);
+  const double flushing = J < 6 ? 1500 : precision_bytes == 8 ? 900 : J == 6 ? 1050 : J == 7 ? 700 : 500;
+  w.grid = pick(dealt, dealt, 0.95, 1, 0, flushing);
   w.normal = pick(2, 2, 0.95, 8, 0.3, 2500);
   return w;
 }

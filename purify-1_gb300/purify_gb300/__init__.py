@@ -71,7 +71,8 @@ class Info(ctypes.Structure):
         ("norm", ctypes.c_double), ("slots", ctypes.c_int64), ("window_cells", ctypes.c_int64),
         ("factor_values", ctypes.c_int64), ("cell_group", ctypes.c_int64),
         ("walk_tasks", ctypes.c_int64), ("walk_steps", ctypes.c_int64),
-        ("row_kernels", ctypes.c_int64),
+        ("row_kernels", ctypes.c_int64), ("degrid_warps", ctypes.c_int64),
+        ("grid_warps", ctypes.c_int64), ("normal_warps", ctypes.c_int64),
     ]
 
 

@@ -35,3 +35,23 @@ def test_chosen_shape_matches_default(pg, cuda, J, dense, precision):
     assert torch.equal(a.adjoint(y), b.adjoint(y))
     tol = 2e-6 if precision == "fp32" else 1e-13
     assert rel_l2(a.normal(x).cpu().numpy(), b.normal(x).cpu().numpy()) < tol
+
+
+@pytest.mark.parametrize("J", [4, 6, 8])
+def test_which_shape_is_chosen(pg, cuda, J):
+    """A few dense tiles take more warps than the default in both directions;
+    coverages whose tiles fill the chip by themselves keep it in G^H (with more it
+    was 1.2 to 1.3 times as slow from J = 6)."""
+    default = 2 if J >= 6 else 4
+
+    def warps(n, M, spread, **kw):
+        rng = np.random.default_rng(J)
+        u, v = (rng.normal(0, spread, M) if spread else rng.uniform(-n, n, M) for _ in range(2))
+        op = pg.MeasurementOperator(np.clip(u, -n, n - 1), np.clip(v, -n, n - 1), None, None, n, n,
+                                    2.0, power_iters=0, kernel="kb", Ju=J, Jv=J, **kw)
+        i = op.info()
+        return i["degrid_warps"], i["grid_warps"], i["normal_warps"]
+    g, gh, normal = warps(64, 60000, 9)
+    assert g > default and gh > default and (normal > 2 if J < 6 else normal == 0)
+    assert warps(400, 200000, 0)[1] == default
+    assert warps(64, 60000, 9, tuning={"threads": 96})[:2] == (3, 3)
