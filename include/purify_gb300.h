@@ -124,8 +124,9 @@ typedef struct {
   int32_t normal_pass;   /* G^H G of purify_gb300_normal and the power method: 1 = one
                             pass over each task where it applies (FP32, unit weights,
                             single-cell items, J <= 6), 2 = degrid then grid through the
-                            slot-ordered buffer, 0 = default (one pass for J < 6); the
-                            results are bit-identical */
+                            slot-ordered buffer, 0 = default (one pass for J < 6); bit-
+                            identical from J = 6 and with equal `threads` (64), else within
+                            rounding (the warp windows are summed in another grouping) */
   int32_t row_kernels;   /* G and G^H of row-factor operators (w rows, supports of 9 to 32,
                             Ju != Jv) in FP32: 1 = the band kernels, 2 = the tensor-core
                             kernels, 3 = G with the former and G^H with the latter (2 and 3

@@ -296,8 +296,7 @@ size_t normal_smem_bytes(int precision_bytes, int J, int win_rows, int win_cols,
 template <typename real, int J, bool SUB>
 cudaError_t launch_normal_one(const ApplyArgs<real> &a, const PolyTable<real> &poly, int ntasks,
                               size_t smem, int threads, cudaStream_t s) {
-  auto fn = a.windows * 32 < threads ? normal_kernel<real, J, SUB, true>
-                                     : normal_kernel<real, J, SUB, false>;
+  auto fn = normal_kernel<real, J, SUB>;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -319,7 +318,6 @@ cudaError_t launch_normal(const ApplyArgs<real> &a, const PolyTable<real> &poly,
     if (ntasks == 0) return cudaSuccess;
     ApplyArgs<real> b = a;
     b.stage_bytes = int(window_bytes(sizeof(real), win_rows, win_cols, shape, false, 1));
-    b.windows = shape.window_count();
     b.win_bytes = b.stage_bytes + int(window_bytes(sizeof(real), win_rows, win_cols, shape, true, 1));
     const bool sub = poly.nsub_u > 1 || poly.nsub_v > 1;
     switch (J) {

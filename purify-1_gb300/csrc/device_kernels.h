@@ -60,8 +60,8 @@ constexpr int kNormBlocks = 512;
 
 struct LaunchShape {
   int threads = 128;  // 32 x warps per CTA
-  // G^H and the normal operator: shared-memory windows of a CTA, a divisor of
-  // its warps (0: one per warp).  See FlushOrder in gridding_device.cuh.
+  // G^H: shared-memory windows of a CTA, a divisor of its warps (0: one per
+  // warp).  See FlushOrder in gridding_device.cuh.
   int windows = 0;
   int window_count() const { return windows > 0 ? windows : threads / 32; }
 };

@@ -687,13 +687,16 @@ __global__ void __launch_bounds__(256) grid_kernel(const ApplyArgs<real> a0,
 // contracts them with F (the visibility degrid_kernel computes, in its order),
 // and adds that value times the taps into the accumulator (grid_kernel's
 // order; the two phase signs cancel).  Null slots add nothing.  Flushes,
-// window sums and the task window written out are grid_kernel's.  So the
-// task windows are those grid_kernel makes from degrid_kernel's slot-ordered
-// output, bit for bit, without the slot-ordered vector and with one tap
-// evaluation per visibility instead of two.  Shared memory: the grid window
+// window sums and the task window written out are grid_kernel's.  So with as
+// many warps as grid_kernel has windows the task windows are those it makes
+// from degrid_kernel's slot-ordered output, bit for bit, without the slot-ordered
+// vector and with one tap evaluation per visibility instead of two.  (With
+// grid_kernel's ordered flushes more warps could share two windows and keep those
+// bits at any support; that took 6% longer than a window per warp on average over
+// 104 coverages, J = 2 to 5.)  Shared memory: the grid window
 // (a.stage_bytes bytes), the warp windows, then the batch headers at
 // a.win_bytes.
-template <typename real, int J, bool SUB, bool ORD>
+template <typename real, int J, bool SUB>
 __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
                                                      const __grid_constant__ PolyTable<real> poly) {
   using C = cplx<real>;
@@ -704,18 +707,17 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   const Task tk = a.tasks[task_id];
   const int WW = tk.W + J - 1, WH = tk.H + J - 1, WS = a.win_stride, WN = win_cells(WH, WS, G);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int nwin = ORD ? a.windows : nw;
   C *gwin = reinterpret_cast<C *>(smem_raw);
   C *wins = reinterpret_cast<C *>(smem_raw + a.stage_bytes);
   const TaskHeaders th = load_headers(a, tk, smem_raw + a.win_bytes);
   {
     // zero the warp windows, 16 bytes per store (stage_bytes is a multiple
     // of 16; an odd FP32 cell count leaves one 8-byte cell at the end)
-    const size_t bytes = size_t(nwin) * WN * sizeof(C);
+    const size_t bytes = size_t(nw) * WN * sizeof(C);
     uint4 *z = reinterpret_cast<uint4 *>(smem_raw + a.stage_bytes);
     for (int idx = threadIdx.x; idx < int(bytes / 16); idx += blockDim.x)
       z[idx] = make_uint4(0u, 0u, 0u, 0u);
-    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nwin * WN - 1] = C{0, 0};
+    if (bytes % 16 != 0 && threadIdx.x == 0) wins[nw * WN - 1] = C{0, 0};
   }
   // tap coefficients of sub-segmented kernels, after the batch headers
   real *csm = reinterpret_cast<real *>(smem_raw + a.win_bytes + kHeaderBytes);
@@ -733,7 +735,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   }
   cp_async_wait_all();
   __syncthreads();
-  C *mine = wins + (ORD ? warp % nwin : warp) * WN;
+  C *mine = wins + warp * WN;
   const int nbt = tk.batch_end - tk.batch_begin;
   const C *frac = static_cast<const C *>(a.frac);
   if (warp < nbt) {
@@ -759,7 +761,6 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
       t1 = stream_load(frac + slot(plb, pk));
       adv(plb, pk);
     }
-    FlushOrder turn(warp, nw, nwin, nbt);
     C F[J][J], acc[J][J];
     int cnt = 0;
     auto load_block = [&](int code) {
@@ -808,7 +809,6 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
         code_n = lane_code_at(th, clb + 2 * nw, nbt, lane);
         const int fcnt = item_count(code);
         C *blk = mine + win_offset(item_lp(code), item_lq(code), WS, G);
-        if constexpr (ORD) turn.wait();
 #pragma unroll
         for (int jv = 0; jv < J; ++jv)
 #pragma unroll
@@ -820,7 +820,6 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
             acc[jv][ju] = C{0, 0};
             __syncwarp();
           }
-        if constexpr (ORD) turn.done();
         adv(clb, ck);
         if (clb < nbt) load_block(code_c);
       } else {
@@ -834,7 +833,7 @@ __global__ void __launch_bounds__(256) normal_kernel(const ApplyArgs<real> a,
   for (int idx = threadIdx.x; idx < WW * WH; idx += blockDim.x, oc.next(WW)) {
     const int e = win_offset(oc.lp, oc.lq, WS, G);
     C s = wins[e];
-    for (int w = 1; w < nwin; ++w) {
+    for (int w = 1; w < nw; ++w) {
       const C o = wins[w * WN + e];
       s.x += o.x;
       s.y += o.y;

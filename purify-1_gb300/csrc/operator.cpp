@@ -46,8 +46,8 @@ namespace {
 // Supports from which the default launch shape and adjoint path change
 // (see the constructor).
 constexpr int kWideSupport = 6;
-// Launch shape of normal_kernel: two windows per CTA (its shared memory holds
-// the grid window besides).
+// Launch shape of normal_kernel, a window per warp beside the grid window: two
+// warps, or more by the plan below kWideSupport (choose_warps).
 constexpr LaunchShape kNormalShape{64};
 // Warps that the batches of a task are dealt to, and windows of a G^H CTA: 4
 // below kWideSupport, 2 from there.
@@ -507,21 +507,22 @@ void OperatorT<real>::init_plain(const OperatorConfig &cfg, int64_t &bytes, Axis
   normal_shape_ = kNormalShape;
   if (cfg.threads == 0 && group_ == 1) {
     // G^H keeps its windows, and with them its bits, whatever its warps
-    // (FlushOrder)
+    // (FlushOrder).  The one-pass normal operator has a window per warp: from
+    // kWideSupport it keeps two, G^H's number, and gives G^H G's bits.
     int optin = 0;
     cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_),
                "cudaDeviceGetAttribute");
     const int nsub = std::max(poly_.nsub_u, poly_.nsub_v);
-    int most = 8;
-    for (; most > rq.warps; most /= 2) {
-      const LaunchShape s{32 * most};
-      if (std::max(degrid_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols, s, true,
-                                     group_, nsub),
-                   normal_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols, s, group_,
-                                     nsub)) <= size_t(optin))
-        break;
-    }
-    const PlanWarps w = choose_warps(plan, rq.warps, most, sizeof(real));
+    int most = 8, most_normal = J_ < kWideSupport ? 8 : 2;
+    while (most > rq.warps &&
+           degrid_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols, LaunchShape{32 * most},
+                             true, group_, nsub) > size_t(optin))
+      most /= 2;
+    while (most_normal > 2 &&
+           normal_smem_bytes(sizeof(real), J_, plan.win_rows, plan.win_cols,
+                             LaunchShape{32 * most_normal}, group_, nsub) > size_t(optin))
+      most_normal /= 2;
+    const PlanWarps w = choose_warps(plan, rq.warps, most, most_normal, sizeof(real));
     degrid_shape_.threads = 32 * w.degrid;
     grid_shape_ = LaunchShape{32 * w.grid, rq.warps};
     normal_shape_.threads = 32 * w.normal;

@@ -123,9 +123,12 @@ void balance_task_batches(Plan &P, int nw) {
 // 512^2 image, 2 x 10^6 visibilities, J = 6: G 65 -> 35 us, G^H 131 -> 77;
 // J = 4: G 39 -> 29, G^H 67 -> 50, normal 90 -> 38.  G takes no fewer warps than
 // the default: on tiles of a batch or two they stage the window more slowly
-// (512^2 image, 6,476 visibilities, Phi: 18.5 us with 4, 20.2 with 2).  From
+// (512^2 image, 6,476 visibilities, Phi: 18.5 us with 4, 20.2 with 2).  The normal
+// operator's margin is the widest: with 5% uniform coverages lost (400^2, 2 x 10^5, J
+// = 5: 49.6 us with 2, 52.9 with 4).  From
 // J = 7 and in FP64 one CTA of 8 warps fills an SM's registers: left out.
-PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) {
+PlanWarps choose_warps(const Plan &P, int dealt, int most, int most_normal,
+                       int precision_bytes) {
   const size_t nt = P.tasks.size();
   std::vector<double> cost(nt);
   for (size_t k = 0; k < nt; ++k) {
@@ -147,12 +150,12 @@ PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) 
     all /= resident;
     return std::max(all, longest) + alpha * std::min(all, longest);
   };
-  auto pick = [&](int usual, int least, double margin, double fixed, double alpha,
+  auto pick = [&](int usual, int most, double margin, double fixed, double alpha,
                   double resident) {
     const double t0 = time(usual, fixed, alpha, resident);
     int best = usual;
     double t = margin * t0;
-    for (int nw = least; nw <= most; nw *= 2)
+    for (int nw = usual; nw <= most; nw *= 2)
       if (nw != usual && time(nw, fixed, alpha, resident) < t) {
         best = nw;
         t = time(nw, fixed, alpha, resident);
@@ -160,10 +163,10 @@ PlanWarps choose_warps(const Plan &P, int dealt, int most, int precision_bytes) 
     return best;
   };
   PlanWarps w;
-  w.degrid = pick(dealt, dealt, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
+  w.degrid = pick(dealt, most, 0.85, J < 5 ? 2 : 5, 0.5, 2000);
   const double flushing = J < 6 ? 1500 : precision_bytes == 8 ? 900 : J == 6 ? 1050 : J == 7 ? 700 : 500;
-  w.grid = pick(dealt, dealt, 0.95, 1, 0, flushing);
-  w.normal = pick(2, 2, 0.95, 8, 0.3, 2500);
+  w.grid = pick(dealt, most, 0.95, 1, 0, flushing);
+  w.normal = pick(2, most_normal, 0.85, 8, 0.3, 2500);
   return w;
 }
 

@@ -113,8 +113,9 @@ PG_HD inline int win_cells(int rows, int WS, int group) {
 }
 
 // Warps per CTA for the gridding kernels on a plan whose batches are dealt to
-// `dealt` warps or windows; at most `most`.
-PlanWarps choose_warps(const Plan &plan, int dealt, int most, int precision_bytes);
+// `dealt` warps or windows; at most `most`, `most_normal` for the normal operator.
+PlanWarps choose_warps(const Plan &plan, int dealt, int most, int most_normal,
+                       int precision_bytes);
 
 // Builds the plan.  Throws std::invalid_argument on bad input.
 Plan build_plan(const PlanRequest &req);

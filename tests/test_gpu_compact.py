@@ -150,3 +150,27 @@ def test_psf_of_non_square_image(pg, oracle_mod, cuda):
     apply_ref, norm_ref = oracle_mod.psf_convolve(oop, ny, nx, 50, 1e-4)
     x = synthetic.sky_image(ny, nx, seed=5)
     assert rel_l2(host(psf(dev(torch, x, "fp64"))), apply_ref(x)) < 1e-10
+
+
+def test_one_pass_normal_keeps_its_promises(pg, cuda):
+    """J = 6, default CTAs, a few dense tiles: the one pass asked for gives the bits
+    of degrid then grid, whose windows are two as well.  And tiles so wide that
+    two windows fit beside the grid window but not four keep the one pass."""
+    torch = cuda
+    rng = np.random.default_rng(3)
+    n, M = 64, 60000
+    u, v = rng.normal(0, 9, M), rng.normal(0, 9, M)
+    a, b = (pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, precision="fp32",
+                                   kernel="kb", Ju=6, Jv=6, tuning={"normal_pass": p})
+            for p in (1, 2))
+    x = dev(torch, synthetic.sky_image(n, n, seed=1), "fp32")
+    assert a.info()["normal_warps"] == 2 and b.info()["normal_warps"] == 0
+    assert torch.equal(a.normal(x), b.normal(x))
+    n = 76  # two tiles of 76 cells an axis
+    x = dev(torch, synthetic.sky_image(n, n, seed=1), "fp32")
+    wide = pg.MeasurementOperator(u, v, None, None, n, n, 2.0, power_iters=0, precision="fp32",
+                                  kernel="kb", Ju=5, Jv=5, tuning={"tile": 76})
+    assert wide.info()["normal_warps"] == 2
+    two = wide.adjoint(wide.forward(x))
+    # another grouping of the window sums: a few roundings
+    assert rel_l2(host(wide.normal(x)), host(two)) < 2e-6
