@@ -131,6 +131,10 @@ typedef struct {
                             Ju != Jv) in FP32: 1 = the band kernels, 2 = the tensor-core
                             kernels, 3 = G with the former and G^H with the latter (2 and 3
                             where supports and scratch allow), 0 = by estimated time */
+  int32_t tap_table;     /* FP64, no row factors: 0 = the tap weights of every visibility are
+                            stored (16 J bytes each) where that takes at most a quarter of
+                            the device memory left free by all else, 1 = never.  The results
+                            are bit-identical */
 } purify_gb300_tuning;
 int purify_gb300_operator_create_tuned(const purify_gb300_create_args *args,
                                        const purify_gb300_tuning *tuning,
@@ -251,6 +255,7 @@ typedef struct {
   int64_t degrid_warps;    /* warps per CTA of G, G^H and the one-pass normal operator (0: two */
   int64_t grid_warps;      /* kernels); 0 for row-factor operators */
   int64_t normal_warps;
+  int64_t tap_table_bytes; /* stored tap weights (FP64), part of device_bytes; 0: none */
 } purify_gb300_info;
 int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_info *info);
 
@@ -376,6 +381,7 @@ typedef struct {
   int32_t cell_group;      /* work-item shape: 1, or 2 (2 x 2) / 3 (row pairs) for FP32, J <= 6 */
   int32_t fft_columns;     /* column transforms of FP32 power-of-two grids: 0 = the library's
                               column pass (grid height <= 2048), 1 = cuFFT's strided plan */
+  int32_t tap_table;       /* FP64: as in purify_gb300_tuning, for all channels or none */
 } purify_gb300_batch_tuning;
 /* Builds the batch (plans every channel, uploads the coverage state).  With
  * tuning == NULL the autotuner picks the tile edge and CTA sizes by timing
@@ -410,6 +416,7 @@ int purify_gb300_batch_get_norms(const purify_gb300_batch *b, double *norms);
 typedef struct {
   int32_t channels, size_groups;
   int64_t visibilities, pixels, tasks, device_bytes;
+  int64_t tap_table_bytes; /* stored tap weights (FP64), part of device_bytes; 0: none */
 } purify_gb300_batch_info;
 int purify_gb300_batch_info_get(const purify_gb300_batch *b, purify_gb300_batch_info *info);
 /* Average device milliseconds of one replay over `reps` replays (after two

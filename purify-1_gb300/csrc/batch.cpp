@@ -433,14 +433,14 @@ BatchT<real>::BatchT(const BatchConfig &cfg) {
   std::vector<size_t> o_taps(nch_);
   if constexpr (sizeof(real) == 8) {
     // stored taps of every channel, or of none (kTapTableShare)
-    size_t total = 0, free_b = 0, total_b = 0;
+    size_t total = 0;
     for (int c = 0; c < nch_; ++c) {
       o_taps[c] = total;
       total += sizeof(real) * 2 * size_t(J_) * size_t(chans_[c].S);
     }
-    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    if (total > 0 && total <= free_b / kTapTableShare) {
-      taps_.alloc(total, &info_.device_bytes);
+    if (cfg.tap_table == 0 && tap_table_fits(total, 0) &&
+        taps_.try_alloc(total, &info_.device_bytes)) {
+      info_.tap_table_bytes = int64_t(total);
       for (int c = 0; c < nch_; ++c)
         cuda_check(launch_tap_table<real>(chans_[c].mem.template at<char>(chans_[c].o_frac), poly_,
                                           J_, chans_[c].S, taps_.as<char>() + o_taps[c], stream_),
@@ -947,6 +947,8 @@ std::unique_ptr<Batch> Batch::create(const BatchConfig &cfg) {
   if (cfg.tile < 8 || cfg.tile > 128) throw Error(kInvalidArgument, "tile must be in [8, 128]");
   if (cfg.max_per_item < 1 || cfg.max_per_item > 64)
     throw Error(kInvalidArgument, "max_per_item must be in [1, 64]");
+  if (cfg.tap_table < 0 || cfg.tap_table > 1)
+    throw Error(kInvalidArgument, "tap_table must be 0 (automatic) or 1 (none)");
   if (cfg.cell_group < 1 || cfg.cell_group > 3)
     throw Error(kInvalidArgument, "cell_group must be 1, 2 or 3");
   if (cfg.cell_group >= 2 && (cfg.fp64 || cfg.J > kMaxGroupJ))

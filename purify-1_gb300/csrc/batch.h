@@ -39,12 +39,14 @@ struct BatchConfig {
   // column transforms of the fused size groups: 0 = launch_fft_cols where it
   // applies, 1 = a strided cuFFT plan
   int fft_columns = 0;
+  int tap_table = 0;  // FP64: 1 = no stored taps
 };
 
 struct BatchInfo {
   int channels = 0;
   int64_t visibilities = 0, pixels = 0, tasks = 0, device_bytes = 0;
   int size_groups = 0;
+  int64_t tap_table_bytes = 0;
   int win_rows = 0, win_cols = 0;  // largest task window over the channels
 };
 
@@ -81,6 +83,7 @@ struct BatchTuning {
   int tile = kTile, max_per_item = 16, degrid_threads = 128, grid_threads = 128;
   int cell_group = 1;
   int fft_columns = 0;
+  int tap_table = 0;
 };
 
 // Picks the uv tile edge, the work-item shape (single cells or 2 x 2 groups)

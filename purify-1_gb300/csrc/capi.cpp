@@ -131,6 +131,7 @@ pg::OperatorConfig to_config(const purify_gb300_create_args *a, const purify_gb3
     c.grid_walk = t->grid_walk;
     c.normal_pass = t->normal_pass;
     c.row_kernels = t->row_kernels;
+    c.tap_table = t->tap_table;
   }
   if (a->precision != PURIFY_GB300_FP32 && a->precision != PURIFY_GB300_FP64)
     throw pg::Error(pg::kInvalidArgument, "unknown precision");
@@ -400,6 +401,7 @@ int purify_gb300_operator_info(const purify_gb300_operator *op, purify_gb300_inf
     info->degrid_warps = i.degrid_warps;
     info->grid_warps = i.grid_warps;
     info->normal_warps = i.normal_warps;
+    info->tap_table_bytes = i.tap_table_bytes;
   });
 }
 
@@ -676,12 +678,14 @@ int purify_gb300_batch_create(const purify_gb300_channel *channels, int32_t nch,
       t.grid_threads = tuning->grid_threads > 0 ? tuning->grid_threads : 128;
       t.cell_group = tuning->cell_group > 0 ? tuning->cell_group : 1;
       t.fft_columns = tuning->fft_columns;
+      t.tap_table = tuning->tap_table;
     } else {
       t = pg::autotune_batch(cfg);
     }
     cfg.tile = t.tile;
     cfg.cell_group = t.cell_group;
     cfg.fft_columns = t.fft_columns;
+    cfg.tap_table = t.tap_table;
     cfg.max_per_item = t.max_per_item;
     cfg.threads = 128;
     cfg.degrid_threads = t.degrid_threads;
@@ -706,6 +710,7 @@ int purify_gb300_batch_get_tuning(const purify_gb300_batch *b, purify_gb300_batc
   t->grid_threads = b->tuning.grid_threads;
   t->cell_group = b->tuning.cell_group;
   t->fft_columns = b->tuning.fft_columns;
+  t->tap_table = b->tuning.tap_table;
   return PURIFY_GB300_OK;
 }
 int purify_gb300_batch_bind(purify_gb300_batch *b, const void *const *x_in, void *const *vis,
@@ -748,6 +753,7 @@ int purify_gb300_batch_info_get(const purify_gb300_batch *b, purify_gb300_batch_
   info->pixels = i.pixels;
   info->tasks = i.tasks;
   info->device_bytes = i.device_bytes;
+  info->tap_table_bytes = i.tap_table_bytes;
   return PURIFY_GB300_OK;
 }
 

@@ -80,9 +80,15 @@ size_t grid_smem_bytes(int precision_bytes, int J, int win_rows, int win_cols,
 // Tap weights of S slots (a multiple of 32) from their fractions, 2 J values
 // per slot in the layout of ApplyArgs::taps, evaluated as the gridding
 // kernels evaluate them, the phase sign folded into the u taps.
-// A table of more than 1 / kTapTableShare of the free device memory is not
-// made; the kernels then evaluate the polynomials, with the same bits.
+// A table is made after all else that its owner allocates, and only within 1 /
+// kTapTableShare of the device memory that is free then; without one the kernels
+// evaluate the polynomials, with the same bits.
 constexpr size_t kTapTableShare = 4;
+inline bool tap_table_fits(size_t bytes, size_t reserve) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
+  return bytes > 0 && free_b > reserve && bytes <= (free_b - reserve) / kTapTableShare;
+}
 template <typename real>
 cudaError_t launch_tap_table(const void *frac, const PolyTable<real> &poly, int J, int64_t S,
                              void *taps, cudaStream_t s);

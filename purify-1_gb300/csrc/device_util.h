@@ -33,6 +33,22 @@ class DeviceBuffer {
     bytes_ = bytes;
     if (counter) *counter += int64_t(bytes);
   }
+  // For memory that the owner can do without: false where there is none.
+  bool try_alloc(size_t bytes, int64_t *counter) {
+    if (cudaMalloc(&p_, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      p_ = nullptr;
+      return false;
+    }
+    bytes_ = bytes;
+    if (counter) *counter += int64_t(bytes);
+    return true;
+  }
+  void reset() {
+    if (p_) cudaFree(p_);
+    p_ = nullptr;
+    bytes_ = 0;
+  }
   void upload(const void *src, size_t bytes, cudaStream_t s) {
     if (bytes) cuda_check(cudaMemcpyAsync(p_, src, bytes, cudaMemcpyHostToDevice, s), "upload");
   }

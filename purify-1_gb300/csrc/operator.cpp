@@ -96,7 +96,12 @@ class OperatorT final : public Operator {
   double power_method(int iters, double tol) override;
   void set_norm(double norm) override;
   double norm() const override { return norm_; }
-  OperatorInfo info() const override { return info_; }
+  OperatorInfo info() const override {
+    std::lock_guard<std::mutex> lock(mu_);  // release_taps
+    OperatorInfo i = info_;
+    i.tap_table_bytes = int64_t(taps_.bytes());
+    return i;
+  }
   void set_stage_timing(bool on) override;
   void stage_times(double *total_ms, int64_t *launches) override;
   WorkspaceSizes workspace_sizes() const override;
@@ -104,6 +109,7 @@ class OperatorT final : public Operator {
   void adjoint_ws(const void *y, void *x, const Workspace &ws) override;
   void power_ws(void *x, int first, int count, double *sq, double *partial,
                 const Workspace &ws) override;
+  bool release_taps() override;
   bool needs_column_plan() const override { return fused_fft_ && !own_cols_; }
 
  private:
@@ -242,9 +248,10 @@ class OperatorT final : public Operator {
   DeviceBuffer tw_v_;
   bool use_fused_fft() const { return fused_fft_ && (own_cols_ || ws_->fft_cols != 0); }
   FftColArgs col_args(const void *in, void *out) const;
-  std::mutex mu_;
+  mutable std::mutex mu_;
 
   DeviceBuffer taps_;  // FP64: stored tap weights of every slot (ApplyArgs::taps)
+  void make_taps(size_t reserve);
   DeviceBuffer task_order_, frac_, weight_, slot_user_, user_slot_, batches_, lane_code_, tasks_, tile_tasks_,
       tu_start_, tv_start_, tu_of_, tv_of_, su_d_, sv_d_, pad_, work_, tilebuf_, slots_,
       norm_partial_, norm_out_;
@@ -471,7 +478,35 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
   }
 
   set_norm(1.0);
+  if (sizeof(real) == 8 && !wmode_ && cfg.tap_table == 0) make_taps(size_t(cfg.tap_reserve));
   if (cfg.power_iters > 0) power_method(cfg.power_iters, cfg.power_tol);
+}
+
+// Stored taps (FP64), 16 J bytes per slot.  Measured on a 512^2 image with
+// 2 x 10^6 visibilities, J = 6: Phi then Phi^H 3142 us with the polynomials, 1700
+// with the table (192 MB; 1070 with the FP64 FFT passes and the launch shapes of
+// today).
+template <typename real>
+void OperatorT<real>::make_taps(size_t reserve) {
+  if constexpr (sizeof(real) == 8) {
+    const size_t bytes = sizeof(real) * 2 * size_t(J_) * size_t(S_);
+    if (!tap_table_fits(bytes, reserve) || !taps_.try_alloc(bytes, &info_.device_bytes)) return;
+    cuda_check(launch_tap_table<real>(frac_.get(), poly_, J_, S_, taps_.get(), stream_),
+               "tap table");
+  }
+}
+
+template <typename real>
+bool OperatorT<real>::release_taps() {
+  DeviceGuard guard(device_);
+  std::lock_guard<std::mutex> lock(mu_);
+  if (!taps_.get()) return false;
+  // launches in flight and recorded ones read the table
+  cuda_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+  drop_graphs();
+  info_.device_bytes -= int64_t(taps_.bytes());
+  taps_.reset();
+  return true;
 }
 
 template <typename real>
@@ -549,20 +584,6 @@ void OperatorT<real>::init_plain(const OperatorConfig &cfg, int64_t &bytes, Axis
   }
   frac_.alloc(sizeof(C) * S_, &bytes);
   frac_.upload(fr.data(), sizeof(C) * S_, stream_);
-  if constexpr (sizeof(real) == 8) {
-    // Stored taps, 16 J bytes per slot.  Measured on a 512^2 image with
-    // 2 x 10^6 visibilities, J = 6: Phi then Phi^H 3142 us with the
-    // polynomials, 1700 with the table (192 MB; 1070 with the FP64 FFT
-    // passes and the launch shapes of today).
-    const size_t tb = sizeof(real) * 2 * size_t(J_) * size_t(S_);
-    size_t free_b = 0, total_b = 0;
-    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    if (S_ > 0 && tb <= free_b / kTapTableShare) {
-      taps_.alloc(tb, &bytes);
-      cuda_check(launch_tap_table<real>(frac_.get(), poly_, J_, S_, taps_.get(), stream_),
-                 "tap table");
-    }
-  }
   std::vector<C> wt;
   if (!unit_weights_) {
     wt.resize(S_);
@@ -1715,6 +1736,8 @@ std::unique_ptr<Operator> Operator::create(const OperatorConfig &cfg) {
   if (cfg.cell_group >= 2 && (cfg.fp64 || cfg.Ju > kMaxGroupJ || cfg.w_term || cfg.Ju != cfg.Jv))
     throw Error(kUnsupported,
                 "2 x 2 and row-pair work items need complex<float>, J <= 6 and no w-projection");
+  if (cfg.tap_table < 0 || cfg.tap_table > 1)
+    throw Error(kInvalidArgument, "tap_table must be 0 (automatic) or 1 (none)");
   if (cfg.row_kernels < 0 || cfg.row_kernels > 3)
     throw Error(kInvalidArgument, "row_kernels must be 0 (automatic), 1, 2 or 3");
   if (cfg.w_term && (cfg.M > 0 && !cfg.w))

@@ -68,6 +68,8 @@ struct OperatorConfig {
   // J = 6, where it measured slower).
   int normal_pass = 0;
   int row_kernels = 0;
+  int tap_table = 0;          // FP64: 1 = no stored taps
+  int64_t tap_reserve = 0;    // device bytes that the stored taps leave free besides
 };
 
 // A plan fraction t + d (see PlanRequest::group) in precision `real`, kept
@@ -93,6 +95,7 @@ struct OperatorInfo {
   int64_t walk_tasks = 0, walk_steps = 0;
   int64_t row_kernels = 0;
   int64_t degrid_warps = 0, grid_warps = 0, normal_warps = 0;
+  int64_t tap_table_bytes = 0;
 };
 
 // Scratch of one apply held outside the operator, so that several applies of
@@ -156,6 +159,10 @@ class Operator {
                         const Workspace &ws) = 0;
   // True when the applies need Workspace::fft_cols (a cuFFT column plan).
   virtual bool needs_column_plan() const = 0;
+  // Gives back the memory of the stored tap weights (FP64; the kernels then
+  // evaluate the polynomials, with the same bits).  Waits for the device.
+  // False where there were none.
+  virtual bool release_taps() = 0;
 };
 
 }  // namespace pg

@@ -175,9 +175,34 @@ Server::~Server() {
   for (auto &kv : pinned_free_) cudaFreeHost(kv.second);
 }
 
+// The stored taps of FP64 coverages (Operator::release_taps) leave the budget
+// free, and make room for what needs memory: a coverage or a request that finds
+// none is tried once more after they are given back.
 int Server::add_coverage(const OperatorConfig &cfg_in) {
   OperatorConfig cfg = cfg_in;
   cfg.device = cfg_.device;
+  cfg.tap_reserve = cfg_.hbm_budget;
+  try {
+    return add_coverage_once(cfg);
+  } catch (const Error &e) {
+    if (e.status != kOutOfMemory || !release_taps()) throw;
+  }
+  cfg.tap_table = 1;
+  return add_coverage_once(cfg);
+}
+
+bool Server::release_taps() {
+  std::vector<Coverage *> all;
+  {
+    std::lock_guard<std::mutex> ck(cov_mu_);
+    for (auto &c : coverages_) all.push_back(c.get());
+  }
+  bool any = false;
+  for (Coverage *c : all) any = c->op->release_taps() || any;
+  return any;
+}
+
+int Server::add_coverage_once(const OperatorConfig &cfg) {
   std::unique_ptr<Coverage> c(new Coverage);
   c->op = Operator::create(cfg);
   c->info = c->op->info();
@@ -451,7 +476,12 @@ bool Server::enqueue(Job &j, cufftHandle fft, cufftHandle fft_cols) {
   Slot &slot = *j.slot;
   cudaStream_t s = slot.stream;
   try {
-    cuda_check(cudaMallocFromPoolAsync(&j.dev, size_t(j.bytes), pool_, s), "request memory");
+    cudaError_t e = cudaMallocFromPoolAsync(&j.dev, size_t(j.bytes), pool_, s);
+    if (e == cudaErrorMemoryAllocation && release_taps()) {
+      cudaGetLastError();
+      e = cudaMallocFromPoolAsync(&j.dev, size_t(j.bytes), pool_, s);
+    }
+    cuda_check(e, "request memory");
     char *p = static_cast<char *>(j.dev);
     auto take = [&](size_t b) {
       char *q = p;

@@ -93,6 +93,8 @@ class Server {
   ServerStats stats() const;
 
  private:
+  int add_coverage_once(const OperatorConfig &cfg);
+  bool release_taps();
   struct Job;
   struct Slot;
   struct Coverage;

@@ -57,7 +57,7 @@ class Tuning(ctypes.Structure):
                 ("cell_group", ctypes.c_int32), ("class_cap", ctypes.c_int32),
                 ("keep_store", ctypes.c_int32), ("fft_columns", ctypes.c_int32),
                 ("grid_walk", ctypes.c_int32), ("normal_pass", ctypes.c_int32),
-                ("row_kernels", ctypes.c_int32)]
+                ("row_kernels", ctypes.c_int32), ("tap_table", ctypes.c_int32)]
 
 
 class Info(ctypes.Structure):
@@ -73,6 +73,7 @@ class Info(ctypes.Structure):
         ("walk_tasks", ctypes.c_int64), ("walk_steps", ctypes.c_int64),
         ("row_kernels", ctypes.c_int64), ("degrid_warps", ctypes.c_int64),
         ("grid_warps", ctypes.c_int64), ("normal_warps", ctypes.c_int64),
+        ("tap_table_bytes", ctypes.c_int64),
     ]
 
 
@@ -91,13 +92,15 @@ class FbParams(ctypes.Structure):
 class BatchTuning(ctypes.Structure):
     _fields_ = [("tile", ctypes.c_int32), ("max_per_item", ctypes.c_int32),
                 ("degrid_threads", ctypes.c_int32), ("grid_threads", ctypes.c_int32),
-                ("cell_group", ctypes.c_int32), ("fft_columns", ctypes.c_int32)]
+                ("cell_group", ctypes.c_int32), ("fft_columns", ctypes.c_int32),
+                ("tap_table", ctypes.c_int32)]
 
 
 class BatchInfo(ctypes.Structure):
     _fields_ = [("channels", ctypes.c_int32), ("size_groups", ctypes.c_int32),
                 ("visibilities", ctypes.c_int64), ("pixels", ctypes.c_int64),
-                ("tasks", ctypes.c_int64), ("device_bytes", ctypes.c_int64)]
+                ("tasks", ctypes.c_int64), ("device_bytes", ctypes.c_int64),
+                ("tap_table_bytes", ctypes.c_int64)]
 
 
 class ServerConfig(ctypes.Structure):
@@ -489,7 +492,7 @@ class MeasurementOperator:
                        int(tuning.get("cell_group", 0)), int(tuning.get("class_cap", 0)),
                        int(tuning.get("keep_store", 0)), int(tuning.get("fft_columns", 0)),
                        int(tuning.get("grid_walk", 0)), int(tuning.get("normal_pass", 0)),
-                       int(tuning.get("row_kernels", 0)))
+                       int(tuning.get("row_kernels", 0)), int(tuning.get("tap_table", 0)))
             _check(L.purify_gb300_operator_create_tuned(ctypes.byref(a), ctypes.byref(t),
                                                         ctypes.byref(h)))
         else:
@@ -711,7 +714,7 @@ class Batch:
             t = BatchTuning(int(tuning.get("tile", 0)), int(tuning.get("max_per_item", 0)),
                             int(tuning.get("degrid_threads", 0)),
                             int(tuning.get("grid_threads", 0)), int(tuning.get("cell_group", 0)),
-                            int(tuning.get("fft_columns", 0)))
+                            int(tuning.get("fft_columns", 0)), int(tuning.get("tap_table", 0)))
         _check(L.purify_gb300_batch_create(arr, n, float(oversample_ratio),
                                            KERNELS[kernel] if isinstance(kernel, str) else int(kernel),
                                            int(J), PRECISIONS[precision], int(device),
@@ -747,7 +750,8 @@ class Batch:
         _check(load().purify_gb300_batch_get_tuning(self._h, ctypes.byref(t)))
         return {"tile": t.tile, "max_per_item": t.max_per_item,
                 "degrid_threads": t.degrid_threads, "grid_threads": t.grid_threads,
-                "cell_group": t.cell_group, "fft_columns": t.fft_columns}
+                "cell_group": t.cell_group, "fft_columns": t.fft_columns,
+                "tap_table": t.tap_table}
 
     def info(self):
         i = BatchInfo()

@@ -51,3 +51,59 @@ def test_stored_taps(pg, oracle_mod, cuda, kernel, J, M, weighted):
     b.apply(2)
     torch.cuda.synchronize()
     assert rel_l2(out[1].cpu().numpy(), a.cpu().numpy()) < 1e-12
+
+
+@pytest.mark.parametrize("kernel,J,n,M", [
+    ("kb", 1, 48, 3000), ("kb", 2, 48, 60000), ("kb", 3, 40, 5000), ("kb", 4, 64, 40000),
+    ("kb", 5, 48, 2000), ("kb", 6, 64, 30000), ("kb", 7, 48, 5000), ("kb", 8, 48, 20000),
+    ("pswf", 6, 40, 9000), ("gauss", 3, 48, 7000), ("kb", 6, 48, 1)])
+def test_table_and_polynomials_give_the_same_bits(pg, cuda, kernel, J, n, M):
+    """tap_table = 1 leaves the table out: forward, adjoint and normal have the
+    same bits either way, for single operators and for a batch."""
+    torch = cuda
+    u, v = synthetic.mixed_uv(M, 2 * n, 2 * n, 0.7, 0.15, seed=J)
+    rng = np.random.default_rng(J)
+    wt = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    kw = dict(power_iters=0, kernel=kernel, Ju=J, Jv=J, precision="fp64")
+    xd = torch.from_numpy(synthetic.sky_image(n, n, seed=J)).cuda()
+    yd = torch.from_numpy(synthetic.random_vis(M, seed=J)).cuda()
+    got, infos = [], []
+    for off in (0, 1):
+        op = pg.MeasurementOperator(u, v, None, wt, n, n, 2.0, tuning={"tap_table": off}, **kw)
+        infos.append(op.info())
+        got.append([op.forward(xd), op.adjoint(yd), op.normal(xd)])
+        b = pg.Batch([dict(u=u, v=v, weights=wt, imsizey=n, imsizex=n)] * 2, kernel=kernel, J=J,
+                     precision="fp64", tuning={"tap_table": off})
+        assert (b.info()["tap_table_bytes"] > 0) == (off == 0)
+        assert b.tuning["tap_table"] == off
+        vis, out = [torch.empty_like(yd) for _ in range(2)], [torch.empty_like(xd) for _ in range(2)]
+        b.bind([xd, xd], vis, out)
+        b.apply(1)
+        torch.cuda.synchronize()
+        got[-1] += [t.clone() for t in vis]
+        for t in vis:
+            t.copy_(yd)
+        b.apply(2)
+        torch.cuda.synchronize()
+        got[-1] += out
+    assert infos[0]["tap_table_bytes"] >= 16 * J * M and infos[1]["tap_table_bytes"] == 0
+    assert (infos[0]["device_bytes"] - infos[1]["device_bytes"] == infos[0]["tap_table_bytes"])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+def test_no_table_in_single_precision_or_where_memory_is_promised(pg, cuda):
+    """FP32 stores no taps; a coverage of a server whose budget is above the free
+    memory stores none either, is built, and gives the same bits."""
+    n, M = 48, 4000
+    u, v = synthetic.mixed_uv(M, 2 * n, 2 * n, 0.7, 0.15, seed=3)
+    args, kw = (u, v, None, None, n, n, 2.0), dict(power_iters=0, Ju=6, Jv=6)
+    assert pg.MeasurementOperator(*args, **kw).info()["tap_table_bytes"] == 0
+    y = synthetic.random_vis(M, seed=3)
+    got = []
+    for budget in (1 << 30, 1 << 45):
+        srv = pg.Server(slots=1, hbm_budget=budget)
+        cov = srv.add_coverage(*args, precision="fp64", **kw)
+        got.append(srv.wait(srv.submit(cov, "adjoint", vis=y)))
+        srv.close()
+    assert np.array_equal(np.asarray(got[0]["x"]), np.asarray(got[1]["x"]))
