@@ -124,8 +124,7 @@ __device__ __forceinline__ void dft(float2 *v) {
 // (S applied) placed at columns x0 ... -> grid row.  Inverse: grid row ->
 // image row (columns x0 ..., S applied).
 template <bool INV>
-__device__ __forceinline__ float2 load_in(const FftArgs &a, const float2 *__restrict__ in, int j,
-                                          int n) {
+__device__ __forceinline__ float2 load_in(const FftArgs &a, const float2 *in, int j, int n) {
   if (j >= a.Ny) return make_float2(0.f, 0.f);
   if constexpr (!INV) {
     const int i = n - a.x0;
@@ -266,12 +265,13 @@ __device__ __forceinline__ void await_twiddles(const TwiddleTable &) {
 // butterfly index read or write one contiguous V x 8-byte row segment; the
 // first stage reads only rows a.y0 ... a.y0+a.Ny-1 (forward), the last writes
 // only those rows (inverse).  Otherwise the first and last stages go through
-// load_in / store_out.
+// load_in / store_out.  No input is __restrict__: a column pass may work in
+// place, and an inverse pass that starts early reads what the kernel ahead of
+// it still writes, so none may be taken for read-only data.
 template <int N, int V, int Ns, int S, bool INV, int PAD = 0, int T = kFftThreads,
           bool COLIO = false, typename TW = TwiddleCache>
-__device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *__restrict__ in,
-                                           float2 *__restrict__ out, float2 *sm,
-                                           const TW &tc, int row0) {
+__device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *in, float2 *out,
+                                           float2 *sm, const TW &tc, int row0) {
   constexpr int R = StageRadix<N, Ns>::value;
   constexpr bool FIRST = Ns == 1, LAST = Ns * R == N;
   constexpr int NB = V * (N / R);  // butterflies of the stage
@@ -332,7 +332,7 @@ __device__ __forceinline__ void run_stages(const FftArgs &a, const float2 *__res
 
 template <int N, int V, bool INV, bool TABLE>
 __global__ void __launch_bounds__(kFftThreads, 4) fft_row_kernel(const FftArgs a,
-                                                              const float2 *__restrict__ in,
+                                                              const float2 *in,
                                                               float2 *__restrict__ out) {
   extern __shared__ float2 fft_sm[];
   dev::pdl_launch_next();
