@@ -91,7 +91,7 @@ constexpr int kOctTerms = 8;
 // block of 8 x 8 cells (row | column << 4), the support S << 8, and how many
 // terms of the same row start here (1 to 3; 0: a later term of a row) << 16.
 // blocks: of its oct, the block rows reached | block columns << 4 | the half
-// of the strip << 8; bit 12: the oct's other four terms are unused.
+// of the strip << 8.
 struct WTerm {
   int64_t a;
   int32_t b_off, m;

@@ -287,7 +287,6 @@ bool build_wstrips(const WPlan &plan, int64_t max_cells, WStripPlan &out) {
     for (int64_t r = first[g]; r < first[g + 1]; ++r) {
       const int32_t i = order[r], code = plan.code[i];
       const int S = wrow_support(code), rank = wrow_rank(code);
-      if (rank == 0) continue;  // no tap is nonzero
       if (used + rank > kOctTerms || half != (key[i] >> 8)) {
         half = key[i] >> 8;
         if (W.octs.size() >= size_t(INT32_MAX) / kOctTerms) return false;
@@ -308,12 +307,11 @@ bool build_wstrips(const WPlan &plan, int64_t max_cells, WStripPlan &out) {
         t.first_tap = start[i] | (S << 8) | ((e == 0 ? rank : 0) << 16);
       }
       used += rank;
-      *oct = tv | (tu << 4) | (half << 8) | (used << 12);
+      *oct = tv | (tu << 4) | (half << 8);
     }
     for (int32_t o = goct[g]; o < int32_t(W.octs.size()); ++o)
       for (int k = 0; k < kOctTerms; ++k)
-        W.terms[size_t(o) * kOctTerms + k].blocks =
-            (W.octs[o] & 0xfff) | (k < 4 && (W.octs[o] >> 12) <= 4 ? 1 << 12 : 0);
+        W.terms[size_t(o) * kOctTerms + k].blocks = W.octs[o];
     goct[g + 1] = int32_t(W.octs.size());
     for (int32_t o = goct[g]; o < goct[g + 1]; ++o)
       cost[g] += int64_t(W.octs[o] & 15) * ((W.octs[o] >> 4) & 15);

@@ -103,7 +103,7 @@ struct WStripPlan {
   std::vector<WStripTask> tasks;     // by strip, then column
   std::vector<int32_t> order;        // launch order: most work first
   std::vector<int32_t> group_oct;    // per task its groups + 1 offsets into octs
-  std::vector<int32_t> octs;         // tv | tu << 4 | half << 8 | terms << 12
+  std::vector<int32_t> octs;         // tv | tu << 4 | half << 8
   std::vector<int64_t> task_cost;    // blocks of a task's octs, and 4 for each group
   std::vector<WTerm> terms;          // 8 per oct
   std::vector<int2_t> owner;         // strips x cols: tasks [x, y) that hold the group

@@ -798,6 +798,7 @@ __global__ void __launch_bounds__(kDegridWarps * 32, 14 / kDegridWarps) wstrip_d
 // rows of one half strip, which the same windows cover but for the last rows
 // of a window, so that one look-up serves eight loads.
 constexpr int kFoldRows = 8;
+static_assert(kStripRows % kFoldRows == 0, "a thread's rows start in one strip");
 __global__ void __launch_bounds__(128) wstrip_fold_kernel(const WStripFoldArgs f) {
   dev::pdl_launch_next();
   dev::pdl_wait();  // the windows are the previous kernel's output
@@ -810,12 +811,11 @@ __global__ void __launch_bounds__(128) wstrip_fold_kernel(const WStripFoldArgs f
   for (int k = 0; k < kFoldRows; ++k) sum[k] = make_float2(0.f, 0.f);
   for (int wv = 0; wv < 2; ++wv) {
     const int pp = p + wv * f.Nv;
-    // strips that reach the first of the rows (with wrapping, rows of an odd
-    // Nv may start a strip between them: such rows are 0 rows of its window)
-    for (int s = min((pp + kFoldRows - 1) / kStripRows, f.strips - 1);
-         s >= 0 && pp - s * kStripRows < f.rows; --s) {
+    // strips that reach the first of the rows; pp >= Nv lies below every strip
+    for (int s = min(pp / kStripRows, f.strips - 1); s >= 0 && pp - s * kStripRows < f.rows;
+         --s) {
       const int r = pp - s * kStripRows;
-      const int k0 = max(0, -r), k1 = min(kFoldRows, f.rows - r);
+      const int k1 = min(kFoldRows, f.rows - r);
       for (int wu = 0; wu < 2; ++wu) {
         const int qq = q + wu * f.Nu;
         int done = -1;  // the last task list summed
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(128) wstrip_fold_kernel(const WStripFoldArgs f
             const int width = __ldg(&f.tasks[n].width);
             const int64_t base = (int64_t(t.y) << 32) | uint32_t(t.x);
             const float2 *v = win + base + int64_t(r) * width + (qq - t.w);
-            if (k0 == 0 && k1 == kFoldRows) {
+            if (k1 == kFoldRows) {
               float2 x[kFoldRows];
 #pragma unroll
               for (int k = 0; k < kFoldRows; ++k) x[k] = __ldcs(v + k * width);
@@ -838,7 +838,7 @@ __global__ void __launch_bounds__(128) wstrip_fold_kernel(const WStripFoldArgs f
             } else {
 #pragma unroll
               for (int k = 0; k < kFoldRows; ++k)
-                if (k >= k0 && k < k1) sum[k] = add2(sum[k], __ldcs(v + k * width));
+                if (k < k1) sum[k] = add2(sum[k], __ldcs(v + k * width));
             }
           }
         }
