@@ -710,8 +710,10 @@ def run_wproj(args):
         "clocks": clocks, "kernel_bytes": wbytes,
         "roofline": roofline_entry(kern, wbytes[kern], dur, peak, peak_kind, None, formula),
         # own kernels per step: the forward row pass, w degrid, w grid, fold,
-        # the inverse row pass (the 4096-row columns go through cuFFT)
-        "gpu_launches": 5 * args.steps,
+        # the inverse row pass; the column passes up to 2048 rows (cuFFT above);
+        # with band kernels in both directions the gathers after G and before G^H
+        "gpu_launches": (5 + (2 if 2 * imsize <= 2048 and args.fft_columns != 1 else 0) +
+                         (2 if info["row_kernels"] == 1 else 0)) * args.steps,
     }
     # FP32 rows against the FP64 oracle on a row sample (rows are independent)
     try:
