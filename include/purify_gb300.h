@@ -116,9 +116,9 @@ typedef struct {
                             (1 .. 16), or 0 for the default */
   int32_t keep_store;    /* 1: Phi's caller-ordered output is stored at L2 evict-last
                             priority (when it fits the L2 share), for a following Phi^H */
-  int32_t fft_columns;   /* column transforms of the FP32 power-of-two FFT path: 0 = the
-                            library's column pass (grid height <= 2048), 1 = cuFFT's
-                            strided column plan */
+  int32_t fft_columns;   /* column transforms of power-of-two grids: 0 = the library's
+                            column pass (grid height <= 2048), 1 = cuFFT's strided column
+                            plan (FP32) or cuFFT for both axes (FP64) */
   int32_t grid_walk;     /* G^H of Phi^H: 1 = the column walk where it applies (tiles <= 32,
                             single-cell items, J <= 8, J <= 6 in FP64), 0 = work items */
   int32_t normal_pass;   /* G^H G of purify_gb300_normal and the power method: 1 = one
@@ -380,7 +380,8 @@ typedef struct {
   int32_t grid_threads;    /* CTA threads of the grouped grid launch */
   int32_t cell_group;      /* work-item shape: 1, or 2 (2 x 2) / 3 (row pairs) for FP32, J <= 6 */
   int32_t fft_columns;     /* column transforms of FP32 power-of-two grids: 0 = the library's
-                              column pass (grid height <= 2048), 1 = cuFFT's strided plan */
+                              column pass (grid height <= 2048), 1 = cuFFT's strided plan
+                              (FP64 batches: cuFFT either way) */
   int32_t tap_table;       /* FP64: as in purify_gb300_tuning, for all channels or none */
 } purify_gb300_batch_tuning;
 /* Builds the batch (plans every channel, uploads the coverage state).  With

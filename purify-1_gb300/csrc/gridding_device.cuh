@@ -301,8 +301,7 @@ __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-//
-// TAB: the taps come from the table at ApplyArgs::taps instead of the
+// degrid_kernel and grid_kernel, TAB: the taps come from the table at ApplyArgs::taps instead of the
 // polynomials.  FP64 kernels are bound by the FP64 pipe (about 1/64 of the
 // FP32 rate): at J = 6 the polynomials are 102 of a visibility's 186 FP64
 // operations per direction.  A table of 96 bytes per slot is read at HBM

@@ -483,9 +483,9 @@ OperatorT<real>::OperatorT(const OperatorConfig &cfg) {
 }
 
 // Stored taps (FP64), 16 J bytes per slot.  Measured on a 512^2 image with
-// 2 x 10^6 visibilities, J = 6: Phi then Phi^H 3142 us with the polynomials, 1700
-// with the table (192 MB; 1070 with the FP64 FFT passes and the launch shapes of
-// today).
+// 2 x 10^6 visibilities, J = 6 (209 MB): Phi 1018 us with the polynomials, 470
+// with the table, Phi^H 1073 and 584.  Made after everything else, so that what
+// is free then is what no other part of the operator needs.
 template <typename real>
 void OperatorT<real>::make_taps(size_t reserve) {
   if constexpr (sizeof(real) == 8) {
