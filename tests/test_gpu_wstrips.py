@@ -1,9 +1,10 @@
 """The tensor-core row kernels (FP32 w-projection rows, supports of 9 to 32
 taps, Ju != Jv) at the edges of their blocks, against the FP64 oracle.
 
-Tolerance (relative L2): 2e-6.  A product keeps about 2^-24 of itself; with
-sums of a few hundred terms of random sign the result is within a few times
-that, 5e-7, and a lost or misplaced tap would show at 1e-3.  Non-finite values stay inside the footprints they belong to;
+Tolerance (relative L2): 2e-6.  Operands are split so that a product keeps
+about 2^-23 of itself; with sums of a few hundred terms of random sign the
+result is within a few times that, 5e-7, and a lost or misplaced tap would
+show at 1e-3.  Non-finite values stay inside the footprints they belong to;
 the finite rest is held to the same tolerance."""
 import numpy as np
 import pytest
