@@ -490,6 +490,8 @@ template <typename real>
 void OperatorT<real>::make_taps(size_t reserve) {
   if constexpr (sizeof(real) == 8) {
     const size_t bytes = sizeof(real) * 2 * size_t(J_) * size_t(S_);
+    // the host entry points' vectors and the power method's, allocated when first used
+    reserve += sizeof(C) * (2 * size_t(N_) + size_t(M_));
     if (!tap_table_fits(bytes, reserve) || !taps_.try_alloc(bytes, &info_.device_bytes)) return;
     cuda_check(launch_tap_table<real>(frac_.get(), poly_, J_, S_, taps_.get(), stream_),
                "tap table");
